@@ -496,8 +496,8 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     ap.add(&c.partials, kMaxPartials);
     c.max_partials = kMaxPartials;
     ap.add(&c.st, 1);
-    ap.add(&c.tw_m, (size_t)c.m / 2);
-    ap.add(&c.tw_n, (size_t)c.n / 2);
+    ap.add(&c.tw_m, c.m);
+    ap.add(&c.tw_n, c.n);
     ap.add(&c.ek_m, c.m);
     ap.add(&c.ek_n, c.n);
     ap.add(&c.wu, c.m);

@@ -234,7 +234,7 @@ struct SpectralPlan {
 };
 void spectral_tables(int m, int n, float bin_w, float bin_h, float2 **tw_m, float2 **tw_n,
                      float2 **ek_m, float2 **ek_n, float **wu, float **wv, cudaStream_t s);
-// The same tables into arrays the caller allocated (m / 2, n / 2, m, n, m, n elements).
+// The same tables into arrays the caller allocated (m, n, m, n, m, n elements).
 void spectral_tables_fill(int m, int n, float bin_w, float bin_h, float2 *tw_m, float2 *tw_n, float2 *ek_m,
                           float2 *ek_n, float *wu, float *wv, cudaStream_t s);
 struct SpectralArgs {
@@ -269,7 +269,6 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
 cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status);
 void dctgemm_destroy(DctGemmPlan *P);
 cudaError_t place_prepare();   // opt the density scatter into its dynamic shared memory
-size_t spectral_smem_bytes(int m, int n);
 
 int ilog2(int v);
 

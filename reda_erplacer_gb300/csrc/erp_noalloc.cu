@@ -32,6 +32,7 @@
 #include <string>
 
 #include "erp_internal.cuh"
+#include "fft_pair.cuh"
 
 namespace erp {
 
@@ -48,8 +49,8 @@ constexpr size_t kOffTx = kOffT1 + kMapBytes;
 constexpr size_t kOffTy = kOffTx + kMapBytes;
 constexpr size_t kOffTp = kOffTy + kMapBytes;
 constexpr size_t kOffTwM = kOffTp + kMapBytes;
-constexpr size_t kOffTwN = kOffTwM + align256(sizeof(float2) * (kMaxSide / 2));
-constexpr size_t kOffEkM = kOffTwN + align256(sizeof(float2) * (kMaxSide / 2));
+constexpr size_t kOffTwN = kOffTwM + align256(sizeof(float2) * kMaxSide);
+constexpr size_t kOffEkM = kOffTwN + align256(sizeof(float2) * kMaxSide);
 constexpr size_t kOffEkN = kOffEkM + align256(sizeof(float2) * kMaxSide);
 constexpr size_t kOffWu = kOffEkN + align256(sizeof(float2) * kMaxSide);
 constexpr size_t kOffWv = kOffWu + align256(sizeof(float) * kMaxSide);
@@ -65,6 +66,13 @@ std::mutex g_setup_mu;
 void *g_scratch_dev[kMaxDevices];
 bool g_ready[kMaxDevices];
 
+// Twiddle t of side N as num / N of a turn, -1 past the table's end: the stage
+// twiddles of the pair FFT (sides 64 and up), W_N^t of the radix-2 one below.
+__device__ int stage_twiddle(int N, int t) {
+    if (N < 64) return t < N / 2 ? t : -1;
+    return t < fft_tw_len(N) ? fft_tw_num(N, t) : -1;
+}
+
 // Twiddle / frequency tables of one (m, n, bin size) and a cleared state block.
 // The trigonometric tables use FP64 sincospi; the frequency vectors repeat the
 // FP32 operations of src/frequencies.rs:10-21.
@@ -72,8 +80,9 @@ __global__ void k_noalloc_tables(int m, int n, float bin_w, float bin_h, float2 
                                  float2 *ek_m, float2 *ek_n, float *wu, float *wv, DevState *st) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     double s, c;
-    if (t < m / 2) { sincospi(-2.0 * t / m, &s, &c); tw_m[t] = make_float2((float)c, (float)s); }
-    if (t < n / 2) { sincospi(-2.0 * t / n, &s, &c); tw_n[t] = make_float2((float)c, (float)s); }
+    const int wm = stage_twiddle(m, t), wn = stage_twiddle(n, t);
+    if (wm >= 0) { sincospi(-2.0 * wm / m, &s, &c); tw_m[t] = make_float2((float)c, (float)s); }
+    if (wn >= 0) { sincospi(-2.0 * wn / n, &s, &c); tw_n[t] = make_float2((float)c, (float)s); }
     if (t < m) {
         sincospi((double)t / (2.0 * m), &s, &c);
         ek_m[t] = make_float2((float)c, (float)-s);

@@ -1,0 +1,35 @@
+"""The spectral solve's buffers: outputs on 4-byte boundaries only take scalar
+stores, and asking for the potential adds blocks to the last pass.  Neither
+changes a bit of the fields, and nothing is written outside the outputs.
+(Accuracy at every side is tested against the oracle in test_gpu_parity.py.)"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n", [(16, 16), (16, 64), (64, 16), (32, 4096), (64, 64), (64, 128), (128, 256), (256, 128),
+                                 (256, 512), (512, 1024), (1024, 512), (2048, 64), (1024, 2048), (4096, 128),
+                                 (128, 4096)])
+def test_solve_buffers(m, n):
+    import torch
+    import reda_erplacer_gb300 as R
+    rng = np.random.default_rng(m * 5 + n)
+    rho = torch.from_numpy((0.7 + 0.3 * rng.random(m * n)).astype(np.float32))
+    s = R.SpectralSolver(m, n, 1.3, 1.0, stream=torch.cuda.current_stream().cuda_stream)
+    results = []
+    for offset in (0, 1, 2):
+        buf = [torch.zeros(m * n + 4, dtype=torch.float32, device="cuda") for _ in range(4)]
+        at = [b[offset:offset + m * n] for b in buf]
+        at[0].copy_(rho)
+        for psi in (at[3].data_ptr(), None):
+            s.solve(at[0].data_ptr(), at[1].data_ptr(), at[2].data_ptr(), psi)
+            torch.cuda.synchronize()
+            results.append([t.clone() for t in at[1:]])
+        for b in buf[1:]:
+            assert float(b[:offset].abs().sum()) == 0 and float(b[offset + m * n:].abs().sum()) == 0
+    s.close()
+    assert float(results[0][0].abs().sum()) > 0 and float(results[0][2].abs().sum()) > 0
+    for r in results[1:]:
+        for a, b in zip(results[0], r):
+            assert torch.equal(a, b)
