@@ -365,13 +365,14 @@ erp_status erp_estimate_footprint(const erp_design *design, const erp_params *pa
  * Mutates the placement state (positions, scheduler): call it after the
  * measured run. */
 typedef enum erp_stage {
-    ERP_STAGE_WIRELENGTH = 0, /* WA nets + HPWL reduction (pin gradients) */
+    ERP_STAGE_WIRELENGTH = 0, /* WA nets + HPWL reduction (pin gradients; whole steps
+                                 finish the HPWL and overflow totals in the Nesterov stage) */
     ERP_STAGE_WL_GATHER = 1,  /* instance gradients from the pin gradients */
     ERP_STAGE_DENSITY = 2,    /* map clear + density scatter */
     ERP_STAGE_SPECTRAL = 3,   /* map conversion + overflow + Poisson solve (3 passes) */
     ERP_STAGE_FORCE = 4,      /* electric force gather (+ the iteration-0 density-weight rescale) */
     ERP_STAGE_NESTEROV = 5,   /* preconditioned gradient / Lipschitz + update */
-    ERP_STAGE_SCHEDULER = 6,
+    ERP_STAGE_SCHEDULER = 6,  /* alone; in whole steps (reps < 0) part of the Nesterov stage */
     ERP_NUM_STAGES = 7
 } erp_stage;
 /* reps > 0: each stage alone, L2 flushed before every launch (mutates the

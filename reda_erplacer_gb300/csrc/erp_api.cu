@@ -261,7 +261,7 @@ SpectralPlan plan_of(Ctx &c) {
 }  // namespace
 
 namespace erp {
-static SpectralArgs spectral_args(Ctx &c, bool zero_map, bool store_rho, bool want_psi) {
+static SpectralArgs spectral_args(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step) {
     SpectralArgs a;
     a.dmap = c.dmap;
     a.initial = c.initial;
@@ -274,13 +274,18 @@ static SpectralArgs spectral_args(Ctx &c, bool zero_map, bool store_rho, bool wa
     a.fx = c.fx;
     a.fy = c.fy;
     a.psi = want_psi ? c.psi : nullptr;
-    a.partials = c.partials;
+    a.partials = step ? c.part_ovf : c.partials;
     a.st = c.st;
+    a.step = step;
     return a;
 }
 
-void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi) {
-    const SpectralArgs a = spectral_args(c, zero_map, store_rho, want_psi);
+int overflow_blocks(const Ctx &c) {
+    return c.gemm ? map_rho_blocks((size_t)c.m * c.n) : spectral_row_blocks(plan_of(const_cast<Ctx &>(c)));
+}
+
+void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step) {
+    const SpectralArgs a = spectral_args(c, zero_map, store_rho, want_psi, step);
     if (c.gemm) {   // tensor-core precisions: rho, then the contractions (rho_out is c.rho itself)
         launch_map_rho(a, (size_t)c.m * c.n, c.rho, c.stream);
         dctgemm_solve(*c.gemm, c.rho, c.fx, c.fy, a.psi, &c.st->status);
@@ -494,6 +499,8 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     float **maps[] = {&c.initial, &c.rho, &c.t1, &c.tx, &c.ty, &c.tp, &c.fx, &c.fy, &c.psi};
     for (float **a : maps) ap.add(a, mn);
     ap.add(&c.partials, kMaxPartials);
+    ap.add(&c.part_wl, kMaxPartials);
+    ap.add(&c.part_ovf, kMaxRowBlocks);
     c.max_partials = kMaxPartials;
     ap.add(&c.st, 1);
     ap.add(&c.tw_m, c.m);
@@ -623,7 +630,7 @@ static erp_status pull_state(Ctx &c) {
 extern "C" erp_status erp_wirelength(erp_ctx *ctx, float gamma, float *hpwl) {
     CTX_CHECK();
     if (!(gamma > 0)) { c.err = "gamma must be positive"; return ERP_EINVAL; }
-    launch_wirelength(c, gamma);
+    launch_wirelength(c, gamma, false);
     launch_wl_gather(c);
     CK(cudaGetLastError());
     if (hpwl) {
@@ -637,7 +644,7 @@ extern "C" erp_status erp_wirelength(erp_ctx *ctx, float gamma, float *hpwl) {
 static void enqueue_potential(Ctx &c, bool stage, bool want_psi) {
     if (stage || c.map_dirty) cudaMemsetAsync(c.dmap, 0, sizeof(unsigned long long) * (size_t)c.m * c.n, c.stream);
     launch_density_scatter(c);
-    launch_spectral(c, /*zero_map=*/!stage, /*store_rho=*/stage, want_psi);
+    launch_spectral(c, /*zero_map=*/!stage, /*store_rho=*/stage, want_psi, /*step=*/false);
     launch_force(c, 0);
     c.map_dirty = stage;
 }
@@ -663,7 +670,7 @@ extern "C" erp_status erp_potential(erp_ctx *ctx, int32_t iteration, float *ener
 extern "C" erp_status erp_nesterov(erp_ctx *ctx, int32_t iteration) {
     CTX_CHECK();
     if (iteration < 0) { c.err = "iteration must be >= 0"; return ERP_EINVAL; }
-    launch_nesterov(c, iteration);
+    launch_nesterov(c, iteration, false);
     CK(cudaGetLastError());
     return ERP_OK;
 }
@@ -687,13 +694,12 @@ extern "C" erp_status erp_should_stop(erp_ctx *ctx, int32_t *stop) {
 namespace erp {
 // Placement::step order (src/placement.rs:180-228)
 void enqueue_step_kernels(Ctx &c) {
-    launch_wirelength(c, -1.0f);
+    launch_wirelength(c, -1.0f, true);
     launch_wl_gather(c);
     launch_density_scatter(c);
-    launch_spectral(c, /*zero_map=*/true, /*store_rho=*/false, /*want_psi=*/false);
+    launch_spectral(c, /*zero_map=*/true, /*store_rho=*/false, /*want_psi=*/false, /*step=*/true);
     launch_force(c, 1);
-    launch_nesterov(c, -1);
-    launch_scheduler(c, 0, 0.f, 0.f);
+    launch_nesterov(c, -1, true);   // with the totals and the scheduler
 }
 }  // namespace erp
 
@@ -1016,19 +1022,18 @@ static erp_status profile_warm(Ctx &c, int reps, float *ms_out) {
     erp_status rc = ERP_OK;
     for (int r = 0; r <= reps && rc == ERP_OK; ++r) {   // r == 0: untimed warm-up
         cudaEventRecord(ev[0], c.stream);
-        launch_wirelength(c, -1.0f);
+        launch_wirelength(c, -1.0f, true);
         cudaEventRecord(ev[1], c.stream);
         launch_wl_gather(c);
         cudaEventRecord(ev[2], c.stream);
         launch_density_scatter(c);
         cudaEventRecord(ev[3], c.stream);
-        launch_spectral(c, /*zero_map=*/true, false, false);
+        launch_spectral(c, /*zero_map=*/true, false, false, true);
         cudaEventRecord(ev[4], c.stream);
         launch_force(c, 1);
         cudaEventRecord(ev[5], c.stream);
-        launch_nesterov(c, -1);
-        cudaEventRecord(ev[6], c.stream);
-        launch_scheduler(c, 0, 0.f, 0.f);
+        launch_nesterov(c, -1, true);
+        cudaEventRecord(ev[6], c.stream);   // the scheduler is part of it
         cudaEventRecord(ev[7], c.stream);
         const cudaError_t err = cudaEventSynchronize(ev[7]);
         if (err != cudaSuccess) {
@@ -1065,15 +1070,15 @@ extern "C" erp_status erp_profile_stages(erp_ctx *ctx, int32_t reps, float *ms_o
             cudaMemsetAsync(flush, r & 0xff, flush_bytes, c.stream);
             cudaEventRecord(e0, c.stream);
             switch (stage) {
-            case ERP_STAGE_WIRELENGTH: launch_wirelength(c, -1.0f); break;
+            case ERP_STAGE_WIRELENGTH: launch_wirelength(c, -1.0f, false); break;
             case ERP_STAGE_WL_GATHER: launch_wl_gather(c); break;
             case ERP_STAGE_DENSITY:
                 cudaMemsetAsync(c.dmap, 0, sizeof(unsigned long long) * mn, c.stream);
                 launch_density_scatter(c);
                 break;
-            case ERP_STAGE_SPECTRAL: launch_spectral(c, true, false, false); break;
+            case ERP_STAGE_SPECTRAL: launch_spectral(c, true, false, false, false); break;
             case ERP_STAGE_FORCE: launch_force(c, 1); break;
-            case ERP_STAGE_NESTEROV: launch_nesterov(c, -1); break;
+            case ERP_STAGE_NESTEROV: launch_nesterov(c, -1, false); break;
             default: launch_scheduler(c, 0, 0.f, 0.f); break;
             }
             cudaEventRecord(e1, c.stream);
@@ -1518,7 +1523,7 @@ static erp_status batch_tune_spectral(erp_batch *b) {
             for (size_t i = 0; i < xs.size(); ++i) {
                 Ctx &x = *xs[i];
                 cudaStreamWaitEvent(x.stream, fork, 0);
-                launch_spectral(x, /*zero_map=*/true, /*store_rho=*/false, /*want_psi=*/false);
+                launch_spectral(x, /*zero_map=*/true, /*store_rho=*/false, /*want_psi=*/false, /*step=*/false);
                 cudaEventRecord(joins[i], x.stream);
                 cudaStreamWaitEvent(b->master, joins[i], 0);
             }
@@ -1602,9 +1607,9 @@ static bool packable(const Ctx &c) {
 static void pack_plan(const std::vector<Ctx *> &xs, PackedArena &ar, std::vector<PackedLaunch> &ls) {
     for (PackKind k : {PK_WA, PK_GATHER, PK_SCATTER}) packed_place_stage(k, xs, ar, ls);
     std::vector<SpectralJob> jobs;
-    for (Ctx *c : xs) jobs.push_back(SpectralJob{plan_of(*c), spectral_args(*c, true, false, false)});
+    for (Ctx *c : xs) jobs.push_back(SpectralJob{plan_of(*c), spectral_args(*c, true, false, false, true)});
     for (PackKind k : {PK_ROWS_DCT_W, PK_COLS_W, PK_ROWS_INV_W}) packed_spectral_stage(k, jobs, ar, ls);
-    for (PackKind k : {PK_FORCE, PK_GRAD, PK_UPDATE, PK_SCHED}) packed_place_stage(k, xs, ar, ls);
+    for (PackKind k : {PK_FORCE, PK_GRAD, PK_UPDATE}) packed_place_stage(k, xs, ar, ls);
 }
 
 static void pack_launch(const std::vector<PackedLaunch> &ls, const void *dev_arena, cudaStream_t s) {
@@ -1892,10 +1897,11 @@ extern "C" erp_status erp_estimate_footprint(const erp_design *d, const erp_para
     auto al = [](int64_t v) { return (v + 511) & ~int64_t(511); };   // allocation granularity
     int64_t b = 16 * al(4 * (N + 4));
     b += al(4 * P) + 2 * al(8 * P) + al(4 * (E + 1)) + al(4 * E) + al(4 * (NM + 1)) + al(4 * movable_pins);
-    b += al(8 * mn) + 9 * al(4 * mn) + al(8 * (int64_t)kMaxPartials) + al(sizeof(DevState));
+    b += al(8 * mn) + 9 * al(4 * mn) + 2 * al(8 * (int64_t)kMaxPartials) +
+         al(8 * (int64_t)kMaxRowBlocks) + al(sizeof(DevState));
     b += 5 * al(4 * (int64_t)NM) + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)scatter_tiles(m, n));   // scatter order
     b += al(4 * (NM + 4)) + al(8 * (NM + 4));   // its inverse, the density gradient in that order
-    b += al(8 * (m / 2)) + al(8 * (n / 2)) + al(8 * m) + al(8 * n) + al(4 * m) + al(4 * n);
+    b += 2 * (al(8 * m) + al(8 * n)) + al(4 * m) + al(4 * n);
     if (pp && pp->precision != ERP_PREC_FP32) {   // tensor-core plan: 4 transforms per axis + 7 map buffers
         const int64_t es = pp->precision == ERP_PREC_TF32_GEMM ? 4 : 4;   // fp32, or bf16 hi + lo
         b += es * (2 * (int64_t)m * m + 2 * (int64_t)n * n + (int64_t)m * m + (int64_t)n * n) + es * 7 * mn;

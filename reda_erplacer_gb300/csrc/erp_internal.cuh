@@ -56,7 +56,9 @@ struct DevState {
 
 constexpr int32_t kStatusWaitTimeout = 2;   // DevState::status bit 1
 
-enum Counter { CTR_HPWL = 0, CTR_OVF = 1, CTR_ABS = 2, CTR_LIP = 3, CTR_ENERGY = 4 };
+// ctr[CTR_UPDATE] is a flag, not a counter: the current step's position update is due
+// (set by k_nesterov_grad, cleared by the step's first kernel).
+enum Counter { CTR_HPWL = 0, CTR_OVF = 1, CTR_ABS = 2, CTR_LIP = 3, CTR_ENERGY = 4, CTR_UPDATE = 7 };
 
 // Net degree classes processed by one thread group of width W each.
 // Classes 0..7 hold nets of one exact degree -- class 0 the leading 2-pin nets
@@ -127,6 +129,7 @@ struct Ctx {
     bool psi_valid;
     // --- reductions ---
     double *partials;          // kMaxPartials
+    double *part_wl, *part_ovf;   // [kMaxPartials], [kMaxRowBlocks]: a step's HPWL and overflow block sums
     int32_t max_partials;
     DevState *st;
     DevState *h_st;            // pinned host mirror
@@ -140,10 +143,13 @@ struct Ctx {
 };
 
 constexpr int kMaxPartials = 8192;
+constexpr int kMaxRowBlocks = 2048;   // 4096 rows, two per block; the map conversion alone: 1,216
 
 // ---------------- launchers (stream = ctx.stream) ----------------
 // wirelength (src/hpwl.rs)
-void launch_wirelength(Ctx &c, float gamma_arg);          // gamma_arg < 0: read DevState.gamma
+// `step` in these launchers: part of a whole step, whose totals and scheduler
+// k_nesterov_update's first block finishes; otherwise each kernel finishes its own total.
+void launch_wirelength(Ctx &c, float gamma_arg, bool step);   // gamma_arg < 0: read DevState.gamma
 void launch_pack_xy(Ctx &c);                               // xy from x, y after a host write
 // headless snapshots (k_snapshot.cu): RGB bytes on the device
 cudaError_t launch_snapshot_placement(Ctx &c, int W, int H, unsigned char *d_rgb, int *d_top);
@@ -153,7 +159,8 @@ void launch_wl_gather(Ctx &c);
 void launch_initial_density(Ctx &c, const float *hx, const float *hy, const float *hw,
                             const float *hh);               // setup, on device
 void launch_density_scatter(Ctx &c);
-void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi);
+void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step);
+int overflow_blocks(const Ctx &c);   // block sums the overflow has in this context's step
 void launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
 int scatter_tiles(int m, int n);
 void launch_xy_from_host(Ctx &c, const float *hx, const float *hy);   // device-mapped host x, y -> x, y, xy
@@ -163,7 +170,7 @@ constexpr int kSortEvery = 16;                          // steps between scatter
 void launch_force(Ctx &c, int rescale);                   // rescale 1: also the iteration-0 density-weight rescale (step graph)
 void launch_energy(Ctx &c);
 // optimiser + scheduler (src/nesterov.rs, src/scheduler.rs)
-void launch_nesterov(Ctx &c, int iter_arg);                // iter_arg < 0: read DevState.iteration
+void launch_nesterov(Ctx &c, int iter_arg, bool step);     // iter_arg < 0: read DevState.iteration
 void launch_scheduler(Ctx &c, int use_args, float hpwl, float overflow);
 // One whole Placement::step on the context's stream (the graph's content).
 void enqueue_step_kernels(Ctx &c);
@@ -202,10 +209,9 @@ inline Packed<P> packed_args(const PackedLaunch &l, const unsigned char *dev) {
     return Packed<P>{reinterpret_cast<const P *>(dev + l.tab), reinterpret_cast<const int32_t *>(dev + l.block0),
                      l.n};
 }
-enum PackKind { PK_WA, PK_GATHER, PK_SCATTER, PK_ROWS_DCT_W, PK_COLS_W, PK_ROWS_INV_W, PK_FORCE, PK_GRAD, PK_UPDATE,
-                PK_SCHED };
+enum PackKind { PK_WA, PK_GATHER, PK_SCATTER, PK_ROWS_DCT_W, PK_COLS_W, PK_ROWS_INV_W, PK_FORCE, PK_GRAD, PK_UPDATE };
 // Appends one packed launch of the given kind over the contexts xs (k_place.cu:
-// wirelength, gather, scatter, force, Nesterov, scheduler; the scatter one per
+// wirelength, gather, scatter, force, Nesterov; the scatter one per
 // plane count in use), and issues a planned launch with the arena at dev (false:
 // not one of its kinds).
 void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &ar, std::vector<PackedLaunch> &out);
@@ -248,7 +254,10 @@ struct SpectralArgs {
     float *fx = nullptr, *fy = nullptr, *psi = nullptr;
     double *partials = nullptr;
     DevState *st = nullptr;
+    bool step = false;                      // part of a whole step: leave the overflow's block sums in partials
 };
+int spectral_row_blocks(const SpectralPlan &p);   // how many those are
+int map_rho_blocks(size_t mn);                    // ... for launch_map_rho
 void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a);
 // The warp-form passes (sides 64..256) of many solves as packed launches, one
 // per template variant in use (k_spectral.cu): kind PK_ROWS_DCT_W, PK_COLS_W or

@@ -256,6 +256,7 @@ struct WaP {
     WaArgs a;
     WaClasses cl;
     float gamma_arg;
+    int step;   // 1: inside a whole step, the block sums are left for the step's tail (k_nesterov_update)
     double * partials;
     DevState * st;
 };
@@ -266,6 +267,7 @@ __device__ __forceinline__ void wa_body(const WaP &p, int bid, int nblk) {
     double *__restrict__ partials = p.partials;
     DevState * st = p.st;
     __shared__ double shr[kThreads / 32];
+    if (p.step && bid == 0 && threadIdx.x == 0) st->ctr[CTR_UPDATE] = 0;   // the step's first kernel
     if (st->done) return;
     const float gamma = gamma_arg > 0.f ? gamma_arg : st->gamma;
     a.inv_gamma = 1.0f / gamma;                        // src/hpwl.rs:166
@@ -293,6 +295,10 @@ __device__ __forceinline__ void wa_body(const WaP &p, int bid, int nblk) {
     }
 #undef ERP_WA_EXACT
     const Df vals[1] = {block_sum(hp, shr)};
+    if (p.step) {
+        leave_partial(partials, bid, vals[0]);
+        return;
+    }
     if (arrive_last(partials, bid, 1, vals, &st->ctr[CTR_HPWL], nblk)) {
         const double tot = sum_partials(partials, nblk, 1, 0, shr);
         if (threadIdx.x == 0) {
@@ -306,6 +312,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wa(const __grid_constant__ WaP 
 
 
 __global__ void k_wl_zero(DevState *st) {
+    if (threadIdx.x == 0) st->ctr[CTR_UPDATE] = 0;   // as k_wa, the step's first kernel
     if (threadIdx.x == 0 && !st->done) {
         st->hpwl = 0.0;
         st->hpwl_f = 0.0f;
@@ -996,6 +1003,7 @@ struct GradP {
     float * pgy;
     double * partials;
     DevState * st;
+    int step;   // 1: inside a whole step, the position update is marked due
 };
 __device__ __forceinline__ void nesterov_grad_body(const GradP &p, int bid, int nblk) {
     int NM = p.NM;
@@ -1015,7 +1023,7 @@ __device__ __forceinline__ void nesterov_grad_body(const GradP &p, int bid, int 
     float *__restrict__ pgy = p.pgy;
     double *__restrict__ partials = p.partials;
     DevState * st = p.st;
-    __shared__ double shr[kThreads / 32];
+    __shared__ double shr[2 * (kThreads / 32)];
     if (st->done) return;
     const float dw = st->dw;
     float numf = 0.0f, denf = 0.0f;
@@ -1044,29 +1052,151 @@ __device__ __forceinline__ void nesterov_grad_body(const GradP &p, int bid, int 
         pgx[i] = gx;
         pgy[i] = gy;
     }
-    Df vals[2];
-    vals[0] = block_sum(numf, shr);
-    vals[1] = block_sum(denf, shr);
-    if (arrive_last(partials, bid, 2, vals, &st->ctr[CTR_LIP], nblk)) {
-        const double tn = sum_partials(partials, nblk, 2, 0, shr);
-        const double td = sum_partials(partials, nblk, 2, 1, shr);
-        if (threadIdx.x == 0) {
-            const int it = iter_arg >= 0 ? iter_arg : st->iteration;
-            const float one = 1.0f, two = one + one, four = two + two;
-            const float a_prev = st->alpha;
-            const float na = (one + sqrtf(four * a_prev * a_prev + one)) / two;
-            st->beta = (a_prev - one) / na;
-            st->alpha = na;
-            if (it > 0 && td > 0.0) st->alpha = (float)sqrt(tn / td);
-            st->lip_num = tn;
-            st->lip_den = td;
-            st->ctr[CTR_LIP] = 0;
-        }
+    Df vals[2] = {Df{numf, 0.0f}, Df{denf, 0.0f}};
+    block_sums(vals, shr);
+    if (!arrive_last(partials, bid, 2, vals, &st->ctr[CTR_LIP], nblk)) return;
+    Df tot[2] = {partials_share(partials, nblk, 2, 0), partials_share(partials, nblk, 2, 1)};
+    block_sums(tot, shr);
+    if (threadIdx.x == 0) {
+        const double tn = df_value(tot[0]), td = df_value(tot[1]);
+        // update_momentum (src/nesterov.rs:148-158), adaptive step length (:98-100)
+        const int it = iter_arg >= 0 ? iter_arg : st->iteration;
+        const float one = 1.0f, two = one + one, four = two + two;
+        const float a_prev = st->alpha;
+        const float na = (one + sqrtf(four * a_prev * a_prev + one)) / two;
+        st->beta = (a_prev - one) / na;
+        st->alpha = it > 0 && td > 0.0 ? (float)sqrt(tn / td) : na;
+        st->lip_num = tn;
+        st->lip_den = td;
+        if (p.step) st->ctr[CTR_UPDATE] = 1;
+        st->ctr[CTR_LIP] = 0;
     }
 }
 __global__ void __launch_bounds__(kThreads) k_nesterov_grad(const __grid_constant__ GradP p) { nesterov_grad_body(p, blockIdx.x, gridDim.x); }
 
 
+// ============================ scheduler ============================
+struct SchedLogs {
+    double ln_shrink, ln_grow, ln_ten;   // ln 0.9999, ln 1.05, ln 10
+};
+
+// Scheduler::update + should_stop (src/scheduler.rs:68-130) in FP64, plus the
+// step record, the non-finite check and the retire-at-overflow flag; one warp, all
+// lanes with the same totals.  The state is loaded up front, so that its latencies
+// overlap the arithmetic.
+__device__ __forceinline__ void run_scheduler(DevState *st, const SchedLogs &lg, float hpwl, float ovf) {
+    const int lane = threadIdx.x & 31;
+    const int it = st->iteration, init_set = st->hpwl_init_set, ovf_set = st->ovf_init_set, stop_iter = st->stop_iter;
+    const float init = st->hpwl_init, prev = st->hpwl_cur, ovf_prev = st->ovf_cur, dw = st->dw, gamma = st->gamma;
+    const float base_gamma = st->base_gamma, alpha = st->alpha, beta = st->beta, stop_overflow = st->stop_overflow;
+    // The density-weight power (lane 0) and the gamma coefficient (lane 1) are
+    // independent FP64 powers of constant bases, b^e = exp(e ln b) with ln b
+    // computed on the host: one convergent exp call evaluates both.  (FP64 runs
+    // at a small fraction of the FP32 rate here; pow's own logarithm was most of
+    // this code's time.)
+    const int it1 = it + 1;
+    const float ref0 = init_set ? init : hpwl;
+    const float delta0 = hpwl - prev;   // hpwl_cur - hpwl_prev after the update below
+    // exponents: (ovf - 0.1) * 20 / 9 - 1 (lane 1), iteration, or -delta / ref,
+    // each as num / den in the same operation order, so one convergent division
+    double lnb, num, den;
+    if (lane == 1) {
+        lnb = lg.ln_ten;
+        num = ((double)ovf - 0.1) * 20.0;
+        den = 9.0;
+    } else if (delta0 < 0.0f) {
+        lnb = lg.ln_shrink;
+        num = (double)it1;
+        den = 1.0;
+    } else {
+        lnb = lg.ln_grow;
+        num = -(double)delta0;
+        den = (double)ref0;
+    }
+    double ex = num / den;
+    if (lane == 1) ex -= 1.0;
+    double pw = exp(ex * lnb);
+    if (lane == 1) pw = pw < 0.05 ? 0.05 : (pw > 10.0 ? 10.0 : pw);
+    else if (delta0 < 0.0f) pw = pw < 0.98 ? 0.98 : pw;
+    else pw = pw < 0.95 ? 0.95 : (pw > 1.05 ? 1.05 : pw);
+    const double coef_l1 = __shfl_sync(0xffffffffu, pw, 1);
+    if (lane != 0) return;
+    erp_step_stats rec;
+    rec.iteration = it;
+    rec.should_stop = (prev != 0.0f && hpwl != 0.0f && prev > hpwl * 1.5f) ? 1 : 0;
+    rec.hpwl = hpwl;
+    rec.overflow = ovf;
+    rec.density_weight = dw;
+    rec.gamma = gamma;
+    rec.alpha = alpha;
+    rec.beta = beta;
+    st->last = rec;
+    st->last_iter = it;
+    st->iteration = it1;
+    if (!init_set) { st->hpwl_init = hpwl; st->hpwl_init_set = 1; }
+    st->hpwl_prev = prev;
+    st->hpwl_cur = hpwl;
+    if (!ovf_set) { st->ovf_init = ovf; st->ovf_init_set = 1; }
+    st->ovf_prev = ovf_prev;
+    st->ovf_cur = ovf;
+    st->dw = (float)((double)dw * (1.05 * pw));
+    st->gamma = (float)((double)base_gamma * coef_l1);
+    const bool bad = !isfinite(hpwl) || !isfinite(ovf) || !isfinite(alpha);
+    if (bad) st->status |= 1;
+    if (bad || (stop_overflow > 0.0f && ovf <= stop_overflow) || (stop_iter > 0 && it1 >= stop_iter)) st->done = 1;
+}
+
+// The scheduler on its own (stage entry points); one warp.
+struct SchedP {
+    int use_args;
+    float hpwl_arg;
+    float ovf_arg;
+    SchedLogs lg;
+    DevState * st;
+};
+__global__ void k_scheduler(const __grid_constant__ SchedP p) {
+    DevState *st = p.st;
+    if (st->done) return;   // warp-uniform
+    run_scheduler(st, p.lg, p.use_args ? p.hpwl_arg : st->hpwl_f, p.use_args ? p.ovf_arg : st->overflow_f);
+}
+
+// Block 0 of a whole step's position update: the HPWL and overflow totals, from the
+// block sums that k_wa and the map conversion left, and the scheduler.  Nothing of
+// the step needs them earlier, and the update's blocks beside it read only alpha,
+// beta and ctr[CTR_UPDATE] (the scheduler may set `done`, with which the update must
+// still run).  A reduction's own tail -- arrival counter, fences, last block's sum --
+// cost 2 to 3 us of kernels that take 3 to 5 at 2,000 cells, and the scheduler's
+// launch 3.3 us; here both hide behind the update.  A step takes 5.6 us less at 2,000
+// and 20,000 cells, 7 us at 200,000 and 8 us at 1M.  (Run by k_nesterov_grad's last
+// block instead, the tail was serial: 9.0 us of gradient pass at 20,000 cells, 5.4 us
+// this way.)
+struct StepTailP {
+    int n_wl, n_ovf;   // block sums of the HPWL and of the overflow
+    const double * part_wl;
+    const double * part_ovf;
+    double movable_area;
+    SchedLogs lg;
+};
+__device__ __forceinline__ void step_tail(const StepTailP &p, DevState *st) {
+    __shared__ double shr[2 * (kThreads / 32)];
+    Df tot[2] = {partials_share(p.part_wl, p.n_wl, 1, 0), partials_share(p.part_ovf, p.n_ovf, 1, 0)};
+    block_sums(tot, shr);
+    if (threadIdx.x >= 32) return;
+    double v[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        v[k] = df_value(Df{__shfl_sync(0xffffffffu, tot[k].hi, 0), __shfl_sync(0xffffffffu, tot[k].lo, 0)});
+    const float hpwl = (float)v[0], ovf = (float)(v[1] / p.movable_area);
+    if (threadIdx.x == 0) {
+        st->hpwl = v[0];
+        st->hpwl_f = hpwl;
+        st->overflow = v[1];
+        st->overflow_f = ovf;
+    }
+    run_scheduler(st, p.lg, hpwl, ovf);
+}
+
+// ============================ position update ============================
 // Lookahead + gradient step + clamp + history (src/nesterov.rs:111-145).
 __device__ __forceinline__ void nesterov_update_cell(float &x, float &y, float &px, float &py, float gx,
                                                      float gy, float w, float h, float die_w, float die_h,
@@ -1098,7 +1228,9 @@ struct UpdateP {
     const float * gx;
     const float * gy;
     float2 * xy;
-    const DevState * st;
+    DevState * st;
+    int step;        // 1: inside a whole step: block 0 runs its tail
+    StepTailP tail;
 };
 __device__ __forceinline__ void nesterov_update_body(const UpdateP &p, int bid, int nblk) {
     int NM = p.NM;
@@ -1113,8 +1245,18 @@ __device__ __forceinline__ void nesterov_update_body(const UpdateP &p, int bid, 
     const float *__restrict__ gx = p.gx;
     const float *__restrict__ gy = p.gy;
     float2 *__restrict__ xy = p.xy;
-    const DevState *__restrict__ st = p.st;
-    if (st->done) return;
+    DevState *st = p.st;
+    if (p.step) {
+        if (st->ctr[CTR_UPDATE] == 0) return;
+        if (bid == 0) {
+            step_tail(p.tail, st);
+            return;
+        }
+        --bid;
+        --nblk;
+    } else if (st->done) {
+        return;
+    }
     const float alpha = st->alpha, beta = st->beta;
     const int n4 = NM >> 2;
     for (int i4 = bid * blockDim.x + threadIdx.x; i4 < n4; i4 += nblk * blockDim.x) {
@@ -1174,95 +1316,6 @@ __global__ void k_xy_to_host(int N, const float2 *__restrict__ xy, float *__rest
     }
 }
 
-// ============================ scheduler ============================
-struct SchedLogs {
-    double ln_shrink, ln_grow, ln_ten;   // ln 0.9999, ln 1.05, ln 10
-};
-
-// Scheduler::update + should_stop (src/scheduler.rs:68-130) in FP64, plus the
-// step record, the non-finite check and the retire-at-overflow flag.
-struct SchedP {
-    int use_args;
-    float hpwl_arg;
-    float ovf_arg;
-    SchedLogs lg;
-    DevState * st;
-};
-__device__ __forceinline__ void scheduler_body(const SchedP &p, int bid, int nblk) {
-    int use_args = p.use_args;
-    float hpwl_arg = p.hpwl_arg;
-    float ovf_arg = p.ovf_arg;
-    SchedLogs lg = p.lg;
-    DevState * st = p.st;
-    if (bid != 0) return;
-    if (st->done) return;   // warp-uniform
-    const float hpwl = use_args ? hpwl_arg : st->hpwl_f;
-    const float ovf = use_args ? ovf_arg : st->overflow_f;
-    // The density-weight power (lane 0) and the gamma coefficient (lane 1) are
-    // independent FP64 powers of constant bases, b^e = exp(e ln b) with ln b
-    // computed on the host: one convergent exp call evaluates both.  (FP64 runs
-    // at a small fraction of the FP32 rate here; pow's own logarithm was most of
-    // this one-warp kernel's time.)
-    const int lane = threadIdx.x & 31;
-    const int it1 = st->iteration + 1;
-    const float ref0 = st->hpwl_init_set ? st->hpwl_init : hpwl;
-    const float delta0 = hpwl - st->hpwl_cur;   // hpwl_cur - hpwl_prev after the update below
-    // exponents: (ovf - 0.1) * 20 / 9 - 1 (lane 1), iteration, or -delta / ref,
-    // each as num / den in the same operation order, so one convergent division
-    double lnb, num, den;
-    if (lane == 1) {
-        lnb = lg.ln_ten;
-        num = ((double)ovf - 0.1) * 20.0;
-        den = 9.0;
-    } else if (delta0 < 0.0f) {
-        lnb = lg.ln_shrink;
-        num = (double)it1;
-        den = 1.0;
-    } else {
-        lnb = lg.ln_grow;
-        num = -(double)delta0;
-        den = (double)ref0;
-    }
-    double ex = num / den;
-    if (lane == 1) ex -= 1.0;
-    double pw = exp(ex * lnb);
-    if (lane == 1) pw = pw < 0.05 ? 0.05 : (pw > 10.0 ? 10.0 : pw);
-    else if (delta0 < 0.0f) pw = pw < 0.98 ? 0.98 : pw;
-    else pw = pw < 0.95 ? 0.95 : (pw > 1.05 ? 1.05 : pw);
-    const double coef_l1 = __shfl_sync(0xffffffffu, pw, 1);
-    if (lane != 0) return;
-    erp_step_stats rec;
-    rec.iteration = st->iteration;
-    rec.hpwl = hpwl;
-    rec.overflow = ovf;
-    rec.density_weight = st->dw;
-    rec.gamma = st->gamma;
-    st->iteration += 1;
-    if (!st->hpwl_init_set) { st->hpwl_init = hpwl; st->hpwl_init_set = 1; }
-    st->hpwl_prev = st->hpwl_cur;
-    st->hpwl_cur = hpwl;
-    if (!st->ovf_init_set) { st->ovf_init = ovf; st->ovf_init_set = 1; }
-    st->ovf_prev = st->ovf_cur;
-    st->ovf_cur = ovf;
-    const double power = pw;   // the rule above, on hpwl_init / hpwl_cur - hpwl_prev / iteration as updated here
-    st->dw = (float)((double)st->dw * (1.05 * power));
-    st->gamma = (float)((double)st->base_gamma * coef_l1);
-    const float cur = st->hpwl_cur, prev = st->hpwl_prev;
-    rec.should_stop = (prev != 0.0f && cur != 0.0f && prev > cur * 1.5f) ? 1 : 0;
-    rec.alpha = st->alpha;
-    rec.beta = st->beta;
-    st->last = rec;
-    st->last_iter = rec.iteration;
-    if (!isfinite(hpwl) || !isfinite(ovf) || !isfinite(st->alpha)) {
-        st->status |= 1;
-        st->done = 1;
-    }
-    if (st->stop_overflow > 0.0f && ovf <= st->stop_overflow) st->done = 1;
-    if (st->stop_iter > 0 && st->iteration >= st->stop_iter) st->done = 1;
-}
-__global__ void k_scheduler(const __grid_constant__ SchedP p) { scheduler_body(p, blockIdx.x, gridDim.x); }
-
-
 __global__ void k_gather_done(DevState *const *states, int count, int32_t *out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
         out[i] = states[i]->done;
@@ -1278,7 +1331,7 @@ static int grid_for(int work, int cap = 152 * 8) {
     return g < 1 ? 1 : (g > cap ? cap : g);
 }
 
-static int wa_params(Ctx &c, float gamma_arg, WaP &p) {
+static int wa_params(Ctx &c, float gamma_arg, bool step, WaP &p) {
     WaArgs a;
     a.net_ptr = c.net_ptr;
     a.slot_cell = c.slot_cell;
@@ -1316,13 +1369,13 @@ static int wa_params(Ctx &c, float gamma_arg, WaP &p) {
         blocks += (int)g;
     }
     cl.block0[kNumClasses] = blocks;
-    p = WaP{a, cl, gamma_arg, c.partials, c.st};
+    p = WaP{a, cl, gamma_arg, step ? 1 : 0, step ? c.part_wl : c.partials, c.st};
     return blocks;
 }
 
-void launch_wirelength(Ctx &c, float gamma_arg) {
+void launch_wirelength(Ctx &c, float gamma_arg, bool step) {
     WaP p;
-    const int blocks = wa_params(c, gamma_arg, p);
+    const int blocks = wa_params(c, gamma_arg, step, p);
     if (blocks == 0) {   // no nets: the total is zero
         k_wl_zero<<<1, 32, 0, c.stream>>>(c.st);
         return;
@@ -1437,18 +1490,32 @@ void launch_energy(Ctx &c) {
         mn, c.psi, c.rho, c.partials, c.st);
 }
 
-static int grad_params(Ctx &c, int iter_arg, GradP &p) {
+// update_density_weight's bases 0.9999 and 1.05, update_gamma's 10
+// (src/scheduler.rs:92-130)
+static SchedLogs sched_logs() {
+    static const SchedLogs lg = {std::log(0.9999), std::log(1.05), std::log(10.0)};
+    return lg;
+}
+
+static int grad_params(Ctx &c, int iter_arg, bool step, GradP &p) {
     p = GradP{c.NM, iter_arg, c.wlgx, c.wlgy, c.dgp, c.pos, c.w, c.h, c.npins, c.x, c.y, c.prev_x, c.prev_y,
-              c.prev_gx, c.prev_gy, c.partials, c.st};
+              c.prev_gx, c.prev_gy, c.partials, c.st, step ? 1 : 0};
     return fit(grid_for((c.NM + 3) / 4), g_res_grad);
 }
 
-static int update_params(Ctx &c, UpdateP &p) {
-    p = UpdateP{c.NM, c.w, c.h, c.die_w, c.die_h, c.x, c.y, c.prev_x, c.prev_y, c.prev_gx, c.prev_gy, c.xy, c.st};
-    return fit(grid_for((c.NM + 3) / 4), g_res_update);
+static int update_params(Ctx &c, bool step, UpdateP &p) {
+    StepTailP tail{};
+    if (step) {
+        WaP w;
+        tail = StepTailP{wa_params(c, -1.0f, true, w), overflow_blocks(c), c.part_wl, c.part_ovf, (double)c.movable_area,
+                         sched_logs()};
+    }
+    p = UpdateP{c.NM, c.w, c.h, c.die_w, c.die_h, c.x, c.y, c.prev_x, c.prev_y, c.prev_gx, c.prev_gy, c.xy, c.st,
+                step ? 1 : 0, tail};
+    return fit(grid_for((c.NM + 3) / 4), g_res_update) + (step ? 1 : 0);
 }
 
-void launch_nesterov(Ctx &c, int iter_arg) {
+void launch_nesterov(Ctx &c, int iter_arg, bool step) {
     if (iter_arg >= 0) {   // stage entry point; in the step graph k_force does the rescale
         const int g = grid_for(c.NM);
         k_dw_rescale<<<g, kThreads, 0, c.stream>>>(c.NM, iter_arg, c.wlgx, c.wlgy, c.dgp, c.pos,
@@ -1456,7 +1523,7 @@ void launch_nesterov(Ctx &c, int iter_arg) {
     }
     GradP pg;
     UpdateP pu;
-    const int gg = grad_params(c, iter_arg, pg), gu = update_params(c, pu);
+    const int gg = grad_params(c, iter_arg, step, pg), gu = update_params(c, step, pu);
     k_nesterov_grad<<<gg, kThreads, 0, c.stream>>>(pg);
     k_nesterov_update<<<gu, kThreads, 0, c.stream>>>(pu);
 }
@@ -1534,15 +1601,8 @@ void launch_xy_to_host(Ctx &c, float *hx, float *hy) {
     k_xy_to_host<<<grid_for(c.N), kThreads, 0, c.stream>>>(c.N, c.xy, hx, hy);
 }
 
-// update_density_weight's bases 0.9999 and 1.05, update_gamma's 10
-// (src/scheduler.rs:92-130)
-static SchedP sched_params(Ctx &c, int use_args, float hpwl, float overflow) {
-    static const SchedLogs lg = {std::log(0.9999), std::log(1.05), std::log(10.0)};
-    return SchedP{use_args, hpwl, overflow, lg, c.st};
-}
-
 void launch_scheduler(Ctx &c, int use_args, float hpwl, float overflow) {
-    k_scheduler<<<1, 32, 0, c.stream>>>(sched_params(c, use_args, hpwl, overflow));
+    k_scheduler<<<1, 32, 0, c.stream>>>(SchedP{use_args, hpwl, overflow, sched_logs(), c.st});
 }
 
 // ---- packed launches (batches) ----
@@ -1574,7 +1634,7 @@ static void plan_stage(PackKind k, int variant, const std::vector<Ctx *> &xs, Pa
 void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &ar, std::vector<PackedLaunch> &out) {
     switch (k) {
     case PK_WA:
-        plan_stage<WaP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, WaP &p) { return wa_params(c, -1.0f, p); });
+        plan_stage<WaP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, WaP &p) { return wa_params(c, -1.0f, true, p); });
         break;
     case PK_GATHER:
         plan_stage<GatherP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, GatherP &p) { return gather_params(c, p); });
@@ -1592,16 +1652,10 @@ void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &a
         plan_stage<ForceP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, ForceP &p) { return force_params(c, 1, p); });
         break;
     case PK_GRAD:
-        plan_stage<GradP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, GradP &p) { return grad_params(c, -1, p); });
+        plan_stage<GradP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, GradP &p) { return grad_params(c, -1, true, p); });
         break;
     case PK_UPDATE:
-        plan_stage<UpdateP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, UpdateP &p) { return update_params(c, p); });
-        break;
-    case PK_SCHED:
-        plan_stage<SchedP>(k, 0, xs, ar, out, 32, 0, [](Ctx &c, SchedP &p) {
-            p = sched_params(c, 0, 0.f, 0.f);
-            return 1;
-        });
+        plan_stage<UpdateP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, UpdateP &p) { return update_params(c, true, p); });
         break;
     default:
         break;
@@ -1641,9 +1695,6 @@ bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaSt
     case PK_UPDATE:
         k_packed<UpdateP, nesterov_update_body, kThreads, 4><<<l.blocks, l.threads, 0, s>>>(
             packed_args<UpdateP>(l, dev));
-        return true;
-    case PK_SCHED:
-        k_packed<SchedP, scheduler_body, 32, 1><<<l.blocks, l.threads, 0, s>>>(packed_args<SchedP>(l, dev));
         return true;
     default:
         return false;

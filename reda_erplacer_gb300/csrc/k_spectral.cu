@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) k_rows_dct_r2(
     const float *__restrict__ rho_in, unsigned long long *__restrict__ dmap,
     const float *__restrict__ initial, float fixed_inv, float coef, float inv_area, int zero_map,
     float *__restrict__ rho_out, float *__restrict__ t1, double *__restrict__ partials,
-    DevState *__restrict__ st, double movable_area) {
+    DevState *__restrict__ st, double movable_area, int step) {
     if (st && st->done) return;
     extern __shared__ __align__(16) float2 sm[];
     float2 *tw = sm;
@@ -131,6 +131,10 @@ __global__ void __launch_bounds__(kThreads) k_rows_dct_r2(
     }
     if (!rho_in && partials) {
         const Df vals[1] = {block_sum(ovf, shr)};
+        if (step) {
+            leave_partial(partials, blockIdx.x, vals[0]);
+            return;
+        }
         if (arrive_last(partials, blockIdx.x, 1, vals, &st->ctr[CTR_OVF], gridDim.x)) {
             const double tot = sum_partials(partials, gridDim.x, 1, 0, shr);
             if (threadIdx.x == 0) {
@@ -379,6 +383,7 @@ struct RowsFwdP {
     double * partials;
     DevState * st;
     double movable_area;
+    int step;   // 1: inside a whole step, the overflow's block sums are left for its tail (k_nesterov_update)
 };
 template <int N, int P>
 __device__ __forceinline__ void rows_fwd_body(const RowsFwdP &a, int bid, int nblk) {
@@ -465,6 +470,10 @@ __device__ __forceinline__ void rows_fwd_body(const RowsFwdP &a, int bid, int nb
     }
     if (from_map && a.partials) {
         const Df vals[1] = {block_sum(ovf, shr)};
+        if (a.step) {
+            leave_partial(a.partials, bid, vals[0]);
+            return;
+        }
         if (arrive_last(a.partials, bid, 1, vals, &st->ctr[CTR_OVF], nblk)) {
             const double tot = sum_partials(a.partials, nblk, 1, 0, shr);
             if (threadIdx.x == 0) {
@@ -669,7 +678,7 @@ __global__ void __launch_bounds__(kThreads) k_map_rho(size_t mn, unsigned long l
                                                       const float *__restrict__ initial, float fixed_inv, float coef,
                                                       float inv_area, int zero_map, float *__restrict__ rho,
                                                       double *__restrict__ partials, DevState *__restrict__ st,
-                                                      double movable_area) {
+                                                      double movable_area, int step) {
     __shared__ double shr[kThreads / 32];
     if (st->done) return;
     Df ovf = df_zero();
@@ -683,6 +692,10 @@ __global__ void __launch_bounds__(kThreads) k_map_rho(size_t mn, unsigned long l
         rho[idx] = __fmul_rn(d, inv_area);         // src/epotential.rs:284-285
     }
     const Df vals[1] = {block_sum(ovf, shr)};
+    if (step) {
+        leave_partial(partials, blockIdx.x, vals[0]);
+        return;
+    }
     if (arrive_last(partials, blockIdx.x, 1, vals, &st->ctr[CTR_OVF], gridDim.x)) {
         const double tot = sum_partials(partials, gridDim.x, 1, 0, shr);
         if (threadIdx.x == 0) {
@@ -693,11 +706,11 @@ __global__ void __launch_bounds__(kThreads) k_map_rho(size_t mn, unsigned long l
     }
 }
 
+int map_rho_blocks(size_t mn) { return (int)std::min<size_t>((mn + kThreads - 1) / kThreads, 152 * 8); }
+
 void launch_map_rho(const SpectralArgs &a, size_t mn, float *rho, cudaStream_t s) {
-    size_t g = (mn + kThreads - 1) / kThreads;
-    if (g > 152 * 8) g = 152 * 8;
-    k_map_rho<<<(int)g, kThreads, 0, s>>>(mn, a.dmap, a.initial, a.fixed_inv, a.coef, a.inv_bin_area,
-                                          a.zero_map ? 1 : 0, rho, a.partials, a.st, a.movable_area);
+    k_map_rho<<<map_rho_blocks(mn), kThreads, 0, s>>>(mn, a.dmap, a.initial, a.fixed_inv, a.coef, a.inv_bin_area,
+                                          a.zero_map ? 1 : 0, rho, a.partials, a.st, a.movable_area, a.step ? 1 : 0);
 }
 
 int ilog2(int v) {
@@ -825,7 +838,7 @@ struct LaunchRowsFwd {
     static RowsFwdP params(const SpectralPlan &p, const SpectralArgs &a) {
         return RowsFwdP{p.m, p.tw_n, p.ek_n, a.rho_in, a.dmap, a.initial, a.fixed_inv, a.coef, a.inv_bin_area,
                         a.zero_map ? 1 : 0, a.rho_out, p.t1, a.rho_in == nullptr ? a.partials : nullptr, a.st,
-                        a.movable_area};
+                        a.movable_area, a.step ? 1 : 0};
     }
     template <int N, int P>
     void operator()() const {
@@ -912,7 +925,7 @@ void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a) {
         k_rows_dct_r2<kRowPairs><<<rb, kThreads, rows_smem(n, kRowPairs), p.stream>>>(
             m, n, p.logn, p.tw_n, p.ek_n, a.rho_in, a.dmap, a.initial, a.fixed_inv, a.coef,
             a.inv_bin_area, a.zero_map ? 1 : 0, a.rho_out, p.t1, from_map ? a.partials : nullptr, a.st,
-            a.movable_area);
+            a.movable_area, a.step ? 1 : 0);
     }
     float *tp = a.psi ? p.tp : nullptr;
     if (pair_side(m)) {
@@ -928,6 +941,19 @@ void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a) {
         k_rows_inv_r2<kRowPairs><<<rb, kThreads, rows_smem(n, kRowPairs), p.stream>>>(
             m, n, p.logn, p.tw_n, p.ek_n, p.tx, p.ty, tp, a.fx, a.fy, a.psi, a.st);
     }
+}
+
+// Blocks of the forward row pass: the overflow's block sums.
+struct RowBlocks {
+    int m;
+    int &blocks;
+    template <int N, int P>
+    void operator()() const { blocks = m / (2 * P); }
+};
+int spectral_row_blocks(const SpectralPlan &p) {
+    int blocks = p.m / (2 * kRowPairs);
+    if (pair_side(p.n)) pair_dispatch<PASS_ROWS_FWD>(p.n, p.seqs, RowBlocks{p.m, blocks});
+    return blocks;
 }
 
 // ---- packed launches of the pair passes (batches) ----
