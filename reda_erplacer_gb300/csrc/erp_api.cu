@@ -392,9 +392,8 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     c.fixed_scale = ldexpf(1.0f, c.shift);
     c.fixed_inv = ldexpf(1.0f, -c.shift);
     {
-        // The scatter keeps each contribution rint((px * py) * 2^S) in 21-bit
-        // pieces; two pieces suffice when no contribution reaches 2^42.  A
-        // contribution is at most ratio * x-overlap * y-overlap * 2^S, an overlap
+        // The scatter keeps each contribution rint((px * py) * 2^S) in pieces of 21
+        // or 23 bits, as few as its bound allows.  A contribution is at most ratio * x-overlap * y-overlap * 2^S, an overlap
         // at most the bin size plus the rounding of a bin edge (a few ulps of the
         // die), the ratio of a movable cell at most 1 (checked here).
         double rmax = 0;
@@ -402,7 +401,9 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
         const double ex = ldexp((double)d->die_w + c.bin_w, -20), ey = ldexp((double)d->die_h + c.bin_h, -20);
         const double cmax = std::max(rmax, 1.0) * ((double)c.bin_w + ex) * ((double)c.bin_h + ey) *
                             ldexp(1.0, c.shift) * (1.0 + ldexp(1.0, -16));
-        c.scatter_planes = cmax < ldexp(1.0, 42) ? 2 : 3;
+        c.scatter_bits = 63;
+        for (int b : {46, 42})
+            if (cmax < ldexp(1.0, b)) c.scatter_bits = b;
     }
     // --- nets: degree classes, internal order, pin slots ---
     std::vector<int> cls_of(E);
@@ -488,7 +489,8 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     ap.add(&c.perm, NM);
     ap.add(&c.pos, (size_t)NM + 4);
     ap.add(&c.dgp, (size_t)NM + 4);
-    ap.add(&c.skey, NM);
+    ap.add(&c.items, scatter_items_max(NM, c.m, c.n));
+    ap.add(&c.n_items, 1);
     ap.add(&c.soff, NM);
     ap.add(&c.sratio, NM);
     ap.add(&c.sort_key, NM);
@@ -562,6 +564,7 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     *c.h_st = h;
     CK(cudaMemcpyAsync(c.st, c.h_st, sizeof(DevState), cudaMemcpyHostToDevice, c.stream));
     launch_pack_xy(c);
+    CK(cudaMemsetAsync(c.n_items, 0, sizeof(int32_t), c.stream));   // without movable cells there are none
     launch_scatter_order(c, c.stream);
     c.sort_age = 0;
     // fixed-cell initial density (src/epotential.rs:127-140)
@@ -1392,13 +1395,24 @@ extern "C" erp_status erp_batch_tuning(const erp_batch *b, int32_t *chosen, int3
 // of the map.  It runs once, at creation (a second calibration after 128
 // iterations, with the cells spread, chose the same shape on the 64-design mix
 // and only cost its time).  ERP_BATCH_SCATTER_CELLS=<n> fixes the choice instead.
+// Every instance's scatter items at `cells` cells, complete on the device on return.
+static erp_status batch_set_scatter(erp_batch *b, int cells) {
+    for (auto *x : b->ctx) {
+        x->c.scatter_cells = cells;
+        launch_scatter_items(x->c, x->c.stream);
+    }
+    for (auto *x : b->ctx)
+        if (cudaStreamSynchronize(x->c.stream) != cudaSuccess)
+            return batch_fail(b, ERP_ECUDA, std::string("scatter items: ") + cudaGetErrorString(cudaGetLastError()));
+    return ERP_OK;
+}
+
 static erp_status batch_tune_scatter(erp_batch *b) {
     const int cand[] = {0, 512, 1024, 2048};
     if (const char *env = getenv("ERP_BATCH_SCATTER_CELLS")) {
         const int v = atoi(env);
         b->scatter_cells = v < 0 ? 0 : std::min(v, 2048);
-        for (auto *x : b->ctx) x->c.scatter_cells = b->scatter_cells;
-        return ERP_OK;
+        return batch_set_scatter(b, b->scatter_cells);
     }
     cudaEvent_t fork, e0, e1;
     if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess) return ERP_ECUDA;
@@ -1411,7 +1425,8 @@ static erp_status batch_tune_scatter(erp_batch *b) {
     erp_status rc = ERP_OK;
     b->tuning.clear();
     for (int c : cand) {
-        for (auto *x : b->ctx) x->c.scatter_cells = c;
+        rc = batch_set_scatter(b, c);
+        if (rc != ERP_OK) break;
         cudaGraph_t g;
         cudaGraphExec_t ge = nullptr;
         cudaError_t e = cudaStreamBeginCapture(b->master, cudaStreamCaptureModeThreadLocal);
@@ -1464,8 +1479,8 @@ static erp_status batch_tune_scatter(erp_batch *b) {
         for (const auto &t : b->tuning)
             if (t.second * 3.0f <= best) best_c = t.first;
     b->scatter_cells = rc == ERP_OK ? best_c : 0;
+    if (rc == ERP_OK) rc = batch_set_scatter(b, b->scatter_cells);
     for (auto *x : b->ctx) {   // the maps are cleared again: the calibration leaves no trace
-        x->c.scatter_cells = b->scatter_cells;
         cudaMemsetAsync(x->c.dmap, 0, sizeof(unsigned long long) * (size_t)x->c.m * x->c.n, b->master);
     }
     if (cudaStreamSynchronize(b->master) != cudaSuccess && rc == ERP_OK) rc = ERP_ECUDA;
@@ -1899,7 +1914,7 @@ extern "C" erp_status erp_estimate_footprint(const erp_design *d, const erp_para
     b += al(4 * P) + 2 * al(8 * P) + al(4 * (E + 1)) + al(4 * E) + al(4 * (NM + 1)) + al(4 * movable_pins);
     b += al(8 * mn) + 9 * al(4 * mn) + 2 * al(8 * (int64_t)kMaxPartials) +
          al(8 * (int64_t)kMaxRowBlocks) + al(sizeof(DevState));
-    b += 5 * al(4 * (int64_t)NM) + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)scatter_tiles(m, n));   // scatter order
+    b += 4 * al(4 * (int64_t)NM) + al(16 * (int64_t)scatter_items_max((int)NM, m, n)) + 512 + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)scatter_tiles(m, n));   // scatter order
     b += al(4 * (NM + 4)) + al(8 * (NM + 4));   // its inverse, the density gradient in that order
     b += 2 * (al(8 * m) + al(8 * n)) + al(4 * m) + al(4 * n);
     if (pp && pp->precision != ERP_PREC_FP32) {   // tensor-core plan: 4 transforms per axis + 7 map buffers
@@ -2038,7 +2053,10 @@ static void server_worker(erp_server *sv) {
             Ctx &c = j->ctx->c;
             // jobs that share the GPU take the batch's scatter shape: fewer, fuller
             // blocks (the shape the batch calibration keeps on the 64-design mix)
-            if (sv->p.max_active > 1) c.scatter_cells = 2048;
+            if (sv->p.max_active > 1) {
+                c.scatter_cells = 2048;
+                launch_scatter_items(c, c.stream);
+            }
             c.h_st->stop_overflow = sv->p.stop_overflow > 0 ? sv->p.stop_overflow : 0.0f;
             c.h_st->stop_iter = sv->p.max_iterations;
             c.h_st->done = 0;

@@ -107,15 +107,18 @@ struct Ctx {
     int32_t *cell_slot_ptr;    // [NM+1]
     int32_t *cell_slots;
     // --- scatter order [NM] (k_density_scatter; refreshed every kSortEvery steps) ---
-    int32_t *perm, *skey;      // cell at each scatter position, its sort tile
+    int32_t *perm;             // cell at each scatter position
+    int4 *items;               // the scatter's work items (cell range, window origin), *n_items of them
+    int32_t *n_items;
     int32_t *pos;              // scatter position of each movable cell (perm's inverse)
     float2 *dgp;               // density gradient in scatter order (k_force writes it coalesced)
     float4 *soff;              // offx, offy, cw, ch in scatter order
     float *sratio;
     int32_t *sort_key, *sort_rank, *sort_hist, *sort_start;   // counting-sort scratch ([NM], [NM], tiles, tiles)
     int32_t sort_age;          // steps since the order was computed
-    int32_t scatter_cells;     // movable cells per scatter block; 0: the rule for a context run alone
-    int32_t scatter_planes;    // 21-bit pieces per contribution in the scatter's window: 2 or 3
+    int32_t scatter_cells;     // movable cells per scatter item; 0: the rule for a context run alone
+                               // (call launch_scatter_items after a change)
+    int32_t scatter_bits;      // every contribution of the scatter is below 2^scatter_bits
     int32_t spectral_seqs;     // sequences per block of the warp-form spectral passes; 0: the fixed shape
     // host-side permutations for test hooks
     int32_t *h_slot_of_pin;    // [P]
@@ -162,7 +165,9 @@ void launch_density_scatter(Ctx &c);
 void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step);
 int overflow_blocks(const Ctx &c);   // block sums the overflow has in this context's step
 void launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
+void launch_scatter_items(Ctx &c, cudaStream_t s);   // its work items again, after scatter_cells changed
 int scatter_tiles(int m, int n);
+int scatter_items_max(int NM, int m, int n);
 void launch_xy_from_host(Ctx &c, const float *hx, const float *hy);   // device-mapped host x, y -> x, y, xy
 void launch_xy_to_host(Ctx &c, float *hx, float *hy);                 // xy -> device-mapped host x, y
 cudaError_t place_occupancy();                        // resident block counts of the streaming kernels
@@ -199,7 +204,7 @@ struct PackedArena {
 };
 struct PackedLaunch {
     int kind;        // PackKind
-    int variant;     // template variant of the kernel (scatter planes; spectral E and NW)
+    int variant;     // template variant of the kernel (scatter pieces; spectral shape)
     size_t tab, block0;   // offsets of the argument table and the block prefix in the arena
     int n, blocks, threads;
     size_t smem;
@@ -212,7 +217,7 @@ inline Packed<P> packed_args(const PackedLaunch &l, const unsigned char *dev) {
 enum PackKind { PK_WA, PK_GATHER, PK_SCATTER, PK_ROWS_DCT_W, PK_COLS_W, PK_ROWS_INV_W, PK_FORCE, PK_GRAD, PK_UPDATE };
 // Appends one packed launch of the given kind over the contexts xs (k_place.cu:
 // wirelength, gather, scatter, force, Nesterov; the scatter one per
-// plane count in use), and issues a planned launch with the arena at dev (false:
+// piece form in use), and issues a planned launch with the arena at dev (false:
 // not one of its kinds).
 void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &ar, std::vector<PackedLaunch> &out);
 bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaStream_t s);

@@ -66,6 +66,39 @@ ERP_FXP_FN uint64_t fxp_rint_u64(float v) {
     return q;
 }
 
+// floor(x 2^-b) for x in [0, 2^(b + 23)) as a float and as an integer, by adding 2^23
+// rounded down; x - floor 2^b exactly.
+ERP_FXP_FN float fxp_high_part(float x, float inv_pow, float pow, uint32_t &high) {
+#if defined(__CUDA_ARCH__)
+    const float t = __fmaf_rd(x, inv_pow, 8388608.0f);
+    high = __float_as_uint(t) - 0x4b000000u;
+    return __fmaf_rn(-__fadd_rn(t, -8388608.0f), pow, x);
+#else
+    const float f = __builtin_floorf(x * inv_pow);   // the product only moves the exponent
+    high = (uint32_t)f;
+    return (float)((double)x - (double)f * (double)pow);
+#endif
+}
+
+// rint(x) (round half to even, as fxp_rint_u64) as s0 + s1 2^B with s0 < 2^B, for x in
+// [0, 2^2B), B = 21..23: nine FP32 and integer instructions and no conversion (those
+// issue at a quarter of the rate).  The low part's own rounding to an integer, by
+// adding 2^23, may reach 2^B and then carries.
+template <int B>
+ERP_FXP_FN void fxp_split2(float x, uint32_t &s0, uint32_t &s1) {
+    static_assert(B >= 21 && B <= 23, "pieces");
+    uint32_t high;
+    const float r = fxp_high_part(x, 1.0f / (float)(1u << B), (float)(1u << B), high);
+    const uint32_t low = fxp_float_bits(r + 8388608.0f) - 0x4b000000u;   // 0 .. 2^B
+    s1 = high + (low >> B);
+    s0 = low & ((1u << B) - 1u);
+}
+// ... as s0 + s1 2^21 + s2 2^42 for x in [0, 2^63).
+ERP_FXP_FN void fxp_split3(float x, uint32_t &s0, uint32_t &s1, uint32_t &s2) {
+    const float r = fxp_high_part(x, 1.0f / 4398046511104.0f, 4398046511104.0f, s2);
+    fxp_split2<21>(r, s0, s1);
+}
+
 // (float)q, round half to even, for any q < 2^64.  The top set bit goes to bit 31
 // of a 32-bit word whose bit 0 also stands for everything below it; that word's
 // own conversion (a native 32-bit one) then rounds as the 64-bit value would, and

@@ -384,15 +384,17 @@ __device__ __forceinline__ float tri_clamped(float x, float s, int k, float bs) 
 // contribution (src/density.rs:195-229), accumulated as rint(v * 2^S) into an
 // int64 map.  Integer sums are order independent, so the privatisation below
 // changes no bit of the result:
-//  * each block owns a kWin x kWin bin window in shared memory anchored at its
-//    first cell; contributions inside it are accumulated there and flushed with
-//    one global atomic per touched bin, the rest go to global memory directly;
-//  * a contribution c in [0, 2^63) is kept in the window as three 21-bit pieces
-//    in three 32-bit planes (32-bit shared atomics are native; 64-bit ones are
-//    several times slower and degrade under contention).  A bin receives at
-//    most one contribution per cell and a block owns at most kMaxCellsPerBlock
-//    = 2^11 cells, so each plane's sum stays below 2^32 and the flush
-//    recombines the exact 64-bit total;
+//  * a block takes an item, a run of cells of one sort tile (below), and owns a
+//    kWin x kWin bin window in shared memory around that tile; contributions
+//    inside it are accumulated there and flushed with one global atomic
+//    per touched bin, the rest go to global memory directly;
+//  * a contribution c in [0, 2^63) is kept in the window in pieces, one 32-bit plane
+//    each (32-bit shared atomics are native; 64-bit ones are several times slower
+//    and degrade under contention): three of 21 bits; two of 21 when c < 2^42; two
+//    of 23 when c < 2^46 and an item holds at most 512 cells.  A bin receives at most
+//    one contribution per cell and an item holds at most kMaxCellsPerBlock = 2^11
+//    cells, so each plane's sum stays below 2^32 and the flush recombines the exact
+//    64-bit total;
 //  * contributions outside the window go to a per-block table of kTable bins
 //    (the slot a bin hashes to, claimed by the first bin that reaches it; a
 //    bin whose slot is taken goes to global memory), so bins that many of the
@@ -403,16 +405,26 @@ __device__ __forceinline__ float tri_clamped(float x, float s, int k, float bs) 
 //
 // Cells are taken in the scatter order (perm, refreshed every few steps by
 // launch_scatter_order): movable cells counting-sorted by a kSortTile-bin square
-// tile of their position, so a block's cells share a tile and its window sits
-// on that tile with kSortPad bins of slack on each side.  Positions come from
+// tile of their position, each tile's cells cut into items of equal size, at most
+// scatter_cap cells.  An item's window sits on its tile with kSortPad bins of slack
+// on each side.  (Blocks of consecutive cells that ignored the tiles' bounds had
+// many cells in the next tile, outside the window.)  The order is up to kSortEvery
+// steps old, and neighbours move together: from kFollowCells cells on, the window
+// sits on the mean position of the item's first 32 cells instead.  Measured: 1M cells
+// over 1024^2 bins, fresh order 41 -> 23 us (per-lane bin loops, 64-bin windows and
+// unaligned blocks before), all cells 20 bins further 41 -> 24 us (39 with the window
+// on the tile); crowded start 31.5 -> 27.7 us.  At 20,000 cells the mean's dependent
+// loads cost 0.5 of 6.6 us.  Tiles of 32 bins (48 before) also bring k_force from
+// 21 to 17 us at 1M cells.  Positions come from
 // the packed xy array; the stretched offsets, sizes and ratios were gathered
 // into the scatter order when it was computed (they never change).  Any
 // permutation gives the same integer sums: the order only decides how many
 // contributions find the window.
-constexpr int kWin = 64;
-constexpr int kSortTile = 48, kSortPad = 8;
+constexpr int kFollowCells = 131072;
+constexpr int kWin = 48;
+constexpr int kSortTile = 32, kSortPad = 8;
 static_assert(kSortTile + 2 * kSortPad == kWin, "the window covers a tile and its pads");
-constexpr int kTableLog = 9, kTable = 1 << kTableLog;   // out-of-window bin table (open, no probing)
+constexpr int kTableLog = 8, kTable = 1 << kTableLog;   // out-of-window bin table (open, no probing)
 constexpr unsigned kEmpty = 0xffffffffu;                 // bin indices are < 4096 * 4096
 constexpr int kMaxCellsPerBlock = 2048;
 // Warp-aggregated scatter for warps whose cells all fall within kAggSide x kAggSide
@@ -422,14 +434,11 @@ constexpr int kMaxCellsPerBlock = 2048;
 // 5 x 5 boxes 4,596 / 4,547 / 4,653 / 4,443 / 4,406 / 4,518: a box takes one warp
 // reduction per bin and plane, which only pays where the warp's cells pile up.
 constexpr int kAggSide = 3;
-constexpr unsigned long long kPiece = (1ull << 21) - 1;
-// Adds the integer s0 + s1 2^21 + s2 2^42 to bin (bx, by): into the block's
+// Adds the integer s0 + s1 2^B (+ s2 2^42) to bin (bx, by): into the block's
 // window plane by plane, else into its bin table, else into global memory.
-// (s0, s1, s2) are the 21-bit pieces of one contribution c = rint((px * py) *
-// 2^S), or their sums over a warp's lanes (each below 2^26).  Every plane's
-// total over a block stays below 2^32: a bin receives at most one contribution
-// per cell, and a block owns at most kMaxCellsPerBlock = 2^11 cells.
-template <int PLANES>
+// (s0, s1, s2) are the pieces of one contribution c = rint((px * py) * 2^S), or their
+// sums over a warp's lanes.
+template <int PLANES, int B>
 __device__ __forceinline__ void scatter_add(int bx, int by, unsigned s0, unsigned s1, unsigned s2, int wox,
                                             int woy, int n, unsigned *win, unsigned *tkey, unsigned *tplane,
                                             unsigned long long *__restrict__ map) {
@@ -455,27 +464,33 @@ __device__ __forceinline__ void scatter_add(int bx, int by, unsigned s0, unsigne
         if (s1) atomicAdd(t + kTable, s1);
         if (PLANES == 3 && s2) atomicAdd(t + 2 * kTable, s2);
     } else {
-        atomicAdd(map + bin, (unsigned long long)s0 + ((unsigned long long)s1 << 21) +
+        atomicAdd(map + bin, (unsigned long long)s0 + ((unsigned long long)s1 << B) +
                                  (PLANES == 3 ? (unsigned long long)s2 << 42 : 0ull));
     }
 }
 
-template <int PLANES>
-__device__ __forceinline__ void scatter_add(int bx, int by, unsigned long long c, int wox, int woy, int n,
-                                            unsigned *win, unsigned *tkey, unsigned *tplane,
-                                            unsigned long long *__restrict__ map) {
-    scatter_add<PLANES>(bx, by, (unsigned)(c & kPiece), (unsigned)((c >> 21) & kPiece),
-                        PLANES == 3 ? (unsigned)(c >> 42) : 0u, wox, woy, n, win, tkey, tplane, map);
+// w += v in shared memory unless v is 0, without a branch (the compiler's own form of
+// `if (v) atomicAdd(...)` diverges and reconverges around every one).
+__device__ __forceinline__ void red_shared_nonzero(unsigned addr, unsigned v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p red.shared.add.u32 [%0], %1;\n\t}" ::"r"(addr), "r"(v)
+                 : "memory");
+}
+
+template <int PLANES, int B>
+__device__ __forceinline__ void scatter_split(float x, unsigned &s0, unsigned &s1, unsigned &s2) {
+    s2 = 0;
+    if (PLANES == 3) fxp_split3(x, s0, s1, s2);
+    else fxp_split2<B>(x, s0, s1);
 }
 
 struct ScatterP {
-    int NM;
     const int32_t * perm;
     const float2 * xy;
     const float4 * soff;
     const float * sratio;
-    const int32_t * skey;
-    int nty;
+    const int4 * items;        // first cell, end, window origin x, y
+    const int32_t * n_items;
+    int follow;                // 1: the window on the cells' current mean position
     int m;
     int n;
     float bw;
@@ -486,15 +501,12 @@ struct ScatterP {
     unsigned long long * map;
     const DevState * st;
 };
-template <int PLANES>
+template <int PLANES, int B>
 __device__ __forceinline__ void density_scatter_body(const ScatterP &p, int bid, int nblk) {
-    int NM = p.NM;
     const int32_t *__restrict__ perm = p.perm;
     const float2 *__restrict__ xy = p.xy;
     const float4 *__restrict__ soff = p.soff;
     const float *__restrict__ sratio = p.sratio;
-    const int32_t *__restrict__ skey = p.skey;
-    int nty = p.nty;
     int m = p.m;
     int n = p.n;
     float bw = p.bw;
@@ -505,119 +517,192 @@ __device__ __forceinline__ void density_scatter_body(const ScatterP &p, int bid,
     unsigned long long *__restrict__ map = p.map;
     const DevState *__restrict__ st = p.st;
     extern __shared__ unsigned dsm[];
-    unsigned *win = dsm;                                  // window planes: bits 0-20, 21-41 (, 42-62)
+    unsigned *win = dsm;                                  // window planes, one per piece
     unsigned *tkey = dsm + PLANES * kWin * kWin;          // bin table: keys (bin index or kEmpty)
     unsigned *tplane = tkey + kTable;                     // bin table: planes
-    {   // shared memory only: overlaps the previous kernel's tail
-        uint4 *w4 = reinterpret_cast<uint4 *>(dsm);
-        for (int k = threadIdx.x; k < PLANES * kWin * kWin / 4; k += blockDim.x) w4[k] = make_uint4(0u, 0u, 0u, 0u);
-        for (int k = threadIdx.x; k < kTable; k += blockDim.x) tkey[k] = kEmpty;
-        for (int k = threadIdx.x; k < PLANES * kTable; k += blockDim.x) tplane[k] = 0u;
-    }
+    const unsigned win_addr = (unsigned)__cvta_generic_to_shared(win);
+    __shared__ int origin[2];
+    // the grid has no more blocks than there can be items, so this one may be read
+    // (and waited for together with the flag and the count) before the count is known
+    int4 it = p.items[bid];
+    const int n_items = *p.n_items;
     if (st->done) return;
-    const int per = ((NM + nblk - 1) / nblk + 31) & ~31;   // <= kMaxCellsPerBlock (launcher)
-    const int c0 = bid * per, c1 = min(c0 + per, NM);
-    int wox = 0, woy = 0;   // window origin: the sort tile of the block's first cell, less the pad
-    if (c0 < NM) {
-        const int k0 = skey[c0];
-        wox = (k0 / nty) * kSortTile - kSortPad;
-        woy = (k0 % nty) * kSortTile - kSortPad;
-    }
-    wox = max(0, min(wox, m - kWin));
-    woy = max(0, min(woy, n - kWin));
-    __syncthreads();
-    for (int base = c0; base < c1; base += blockDim.x) {
-        const int p = base + threadIdx.x;
-        int bxl = 0, byl = 0, nx = 0, ny = 0;
-        float xi = 0.f, yi = 0.f, sxi = 0.f, syi = 0.f, r = 0.f;
-        if (p < c1) {
-            const float2 q = xy[perm[p]];
-            const float4 o = soff[p];   // offx, offy, cw, ch of cell perm[p]
-            xi = q.x + o.x;
-            yi = q.y + o.y;
-            sxi = o.z;
-            syi = o.w;
-            r = sratio[p];
-            int xl = (int)floorf(clamp_bin((xi - 0.0f) * inv_bw, m));
-            int xh = (int)ceilf(clamp_bin((xi - 0.0f + sxi) * inv_bw, m)) + 1;
-            int yl = (int)floorf(clamp_bin((yi - 0.0f) * inv_bh, n));
-            int yh = (int)ceilf(clamp_bin((yi - 0.0f + syi) * inv_bh, n)) + 1;
-            xl = max(xl, 0); xh = min(xh, m - 1);
-            yl = max(yl, 0); yh = min(yh, n - 1);
-            bxl = xl; byl = yl;
-            nx = max(xh - xl, 0);
-            ny = max(yh - yl, 0);
-        }
-        // the bins the warp's cells reach together (their full ranges)
-        const unsigned full = 0xffffffffu;
-        const bool any = nx > 0 && ny > 0;
-        const int ax = __reduce_min_sync(full, any ? bxl : INT_MAX);
-        const int ay = __reduce_min_sync(full, any ? byl : INT_MAX);
-        const int ex = __reduce_max_sync(full, any ? bxl + nx : INT_MIN);
-        const int ey = __reduce_max_sync(full, any ? byl + ny : INT_MIN);
-        if (ax != INT_MAX && ex - ax <= kAggSide && ey - ay <= kAggSide) {
-            // Warp-aggregated atomics.  The warp's cells crowd into at most
-            // kAggSide x kAggSide bins (early in the run most cells sit within a
-            // few bins of the die centre).  Bin by bin, every lane forms its
-            // contribution -- zero outside its own range -- the warp sums the
-            // 21-bit pieces, and one lane adds the sums: one atomic per bin and
-            // plane instead of up to 32 contending ones.  Integer sums, so the
-            // bits are those of the lanes' own adds.
-            const int lane = threadIdx.x & 31;
-            float pyk[kAggSide];
-#pragma unroll
-            for (int k = 0; k < kAggSide; ++k) {
-                const int by = ay + k;
-                pyk[k] = (by >= byl && by < byl + ny) ? tri_clamped(yi, syi, by, bh) : 0.0f;
+    for (int item = bid; item < n_items; item += nblk) {
+        if (item != bid) it = p.items[item];
+        const int c0 = it.x, c1 = it.y;
+        int wox = it.z, woy = it.w;
+        if (p.follow && threadIdx.x < 32) {   // the mean bin of the item's first cells, now
+            const int cnt = min(c1 - c0, 32);
+            int bx = 0, by = 0;
+            if ((int)threadIdx.x < cnt) {
+                const float2 q = xy[perm[c0 + threadIdx.x]];
+                bx = (int)clamp_bin(q.x * inv_bw, m);
+                by = (int)clamp_bin(q.y * inv_bh, n);
             }
-            for (int bx = ax; bx < ex; ++bx) {
-                const float px = (bx >= bxl && bx < bxl + nx) ? r * tri_clamped(xi, sxi, bx, bw) : 0.0f;
+            bx = __reduce_add_sync(0xffffffffu, bx) / cnt;
+            by = __reduce_add_sync(0xffffffffu, by) / cnt;
+            if (threadIdx.x == 0) {
+                origin[0] = max(0, min(bx + 1 - kWin / 2, m - kWin));
+                origin[1] = max(0, min(by + 1 - kWin / 2, n - kWin));
+            }
+        }
+        {
+            uint4 *w4 = reinterpret_cast<uint4 *>(dsm);
+            for (int k = threadIdx.x; k < PLANES * kWin * kWin / 4; k += blockDim.x) w4[k] = make_uint4(0u, 0u, 0u, 0u);
+            for (int k = threadIdx.x; k < kTable; k += blockDim.x) tkey[k] = kEmpty;
+            for (int k = threadIdx.x; k < PLANES * kTable; k += blockDim.x) tplane[k] = 0u;
+        }
+        __syncthreads();
+        if (p.follow) {
+            wox = origin[0];
+            woy = origin[1];
+        }
+        for (int base = c0; base < c1; base += blockDim.x) {
+            int bxl = 0, byl = 0, nx = 0, ny = 0;
+            float xi = 0.f, yi = 0.f, sxi = 0.f, syi = 0.f, ri = 0.f;
+            const int at = base + (int)threadIdx.x;
+            if (at < c1) {
+                const float2 q = xy[perm[at]];
+                const float4 o = soff[at];   // offx, offy, cw, ch of cell perm[at]
+                ri = sratio[at];
+                xi = q.x + o.x;
+                yi = q.y + o.y;
+                sxi = o.z;
+                syi = o.w;
+                int xl = (int)floorf(clamp_bin((xi - 0.0f) * inv_bw, m));
+                int xh = (int)ceilf(clamp_bin((xi - 0.0f + sxi) * inv_bw, m)) + 1;
+                int yl = (int)floorf(clamp_bin((yi - 0.0f) * inv_bh, n));
+                int yh = (int)ceilf(clamp_bin((yi - 0.0f + syi) * inv_bh, n)) + 1;
+                xl = max(xl, 0); xh = min(xh, m - 1);
+                yl = max(yl, 0); yh = min(yh, n - 1);
+                bxl = xl; byl = yl;
+                nx = max(xh - xl, 0);
+                ny = max(yh - yl, 0);
+            }
+            // the bins the warp's cells reach together (their full ranges)
+            const unsigned full = 0xffffffffu;
+            const bool any = nx > 0 && ny > 0;
+            const int ax = __reduce_min_sync(full, any ? bxl : INT_MAX);
+            const int ay = __reduce_min_sync(full, any ? byl : INT_MAX);
+            const int ex = __reduce_max_sync(full, any ? bxl + nx : INT_MIN);
+            const int ey = __reduce_max_sync(full, any ? byl + ny : INT_MIN);
+            if (ax != INT_MAX && ex - ax <= kAggSide && ey - ay <= kAggSide) {
+                // Warp-aggregated atomics.  The warp's cells crowd into at most
+                // kAggSide x kAggSide bins (early in the run most cells sit within a
+                // few bins of the die centre).  Bin by bin, every lane forms its
+                // contribution -- zero outside its own range -- the warp sums the
+                // pieces, and one lane adds the sums: one atomic per bin and
+                // plane instead of up to 32 contending ones.  Integer sums, so the
+                // bits are those of the lanes' own adds.
+                const int lane = threadIdx.x & 31;
+                float pyk[kAggSide];
 #pragma unroll
                 for (int k = 0; k < kAggSide; ++k) {
-                    if (ay + k < ey) {   // warp-uniform
-                        const unsigned long long c = (unsigned long long)fxp_rint_u64((px * pyk[k]) * scale);
-                        const unsigned s0 = __reduce_add_sync(full, (unsigned)(c & kPiece));
-                        const unsigned s1 = __reduce_add_sync(full, (unsigned)((c >> 21) & kPiece));
-                        const unsigned s2 = PLANES == 3 ? __reduce_add_sync(full, (unsigned)(c >> 42)) : 0u;
-                        if (lane == 0 && (s0 | s1 | s2))
-                            scatter_add<PLANES>(bx, ay + k, s0, s1, s2, wox, woy, n, win, tkey, tplane, map);
+                    const int by = ay + k;
+                    pyk[k] = (by >= byl && by < byl + ny) ? tri_clamped(yi, syi, by, bh) : 0.0f;
+                }
+                for (int bx = ax; bx < ex; ++bx) {
+                    const float px = (bx >= bxl && bx < bxl + nx) ? ri * tri_clamped(xi, sxi, bx, bw) : 0.0f;
+#pragma unroll
+                    for (int k = 0; k < kAggSide; ++k) {
+                        if (ay + k < ey) {   // warp-uniform
+                            unsigned s0, s1, s2;
+                            scatter_split<PLANES, B>((px * pyk[k]) * scale, s0, s1, s2);
+                            s0 = __reduce_add_sync(full, s0);
+                            s1 = __reduce_add_sync(full, s1);
+                            if (PLANES == 3) s2 = __reduce_add_sync(full, s2);
+                            if (lane == 0 && (s0 | s1 | s2))
+                                scatter_add<PLANES, B>(bx, ay + k, s0, s1, s2, wox, woy, n, win, tkey, tplane, map);
+                        }
+                    }
+                }
+                continue;
+            }
+            // A cell covers at most three bins an axis when its end lies at or before the
+            // fourth bin's edge: every later overlap is then 0 (its lower bound is not
+            // below that edge).  True of all cells narrower than two bins, since the
+            // stretched size is the larger of the cell's and sqrt(2) bins.
+            const float ex3 = xi + sxi, ey3 = yi + syi;
+            const bool three = (nx <= 3 || ex3 <= 0.0f + (float)(bxl + 3) * bw) && (ny <= 3 || ey3 <= 0.0f + (float)(byl + 3) * bh);
+            if (__all_sync(full, three)) {
+                // spread cells, unrolled: three overlaps an axis, nine contributions, no
+                // loop that lanes leave at different bins
+                float px[3], py[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    px[k] = k < nx ? ri * tri_clamped(xi, sxi, bxl + k, bw) : 0.0f;
+                    py[k] = k < ny ? tri_clamped(yi, syi, byl + k, bh) : 0.0f;
+                }
+                const unsigned wx = (unsigned)(bxl - wox), wy = (unsigned)(byl - woy);
+                const bool inside = wx <= (unsigned)(kWin - 3) && wy <= (unsigned)(kWin - 3);   // all nine bins
+                if (__all_sync(full, inside || !any)) {
+                    const unsigned w = win_addr + 4u * (inside ? wx * kWin + wy : 0u);
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                        for (int dy = 0; dy < 3; ++dy) {
+                            unsigned s0, s1, s2;
+                            scatter_split<PLANES, B>((px[dx] * py[dy]) * scale, s0, s1, s2);
+                            const unsigned at = w + 4u * (dx * kWin + dy);
+                            red_shared_nonzero(at, s0);
+                            red_shared_nonzero(at + 4u * kWin * kWin, s1);
+                            if (PLANES == 3) red_shared_nonzero(at + 8u * kWin * kWin, s2);
+                        }
+                } else {
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                        for (int dy = 0; dy < 3; ++dy) {
+                            unsigned s0, s1, s2;
+                            scatter_split<PLANES, B>((px[dx] * py[dy]) * scale, s0, s1, s2);
+                            if (s0 | s1 | s2)
+                                scatter_add<PLANES, B>(bxl + dx, byl + dy, s0, s1, s2, wox, woy, n, win, tkey, tplane, map);
+                        }
+                }
+            } else {
+                // wide cells among them: each lane its own bin columns and rows
+                for (int dx = 0; dx < nx; ++dx) {
+                    const int bx = bxl + dx;
+                    const float px = ri * tri_clamped(xi, sxi, bx, bw);
+                    if (px == 0.0f) continue;   // every contribution of this bin column is 0
+                    for (int dy = 0; dy < ny; ++dy) {
+                        const int by = byl + dy;
+                        const float py = tri_clamped(yi, syi, by, bh);
+                        unsigned s0, s1, s2;
+                        scatter_split<PLANES, B>((px * py) * scale, s0, s1, s2);
+                        if (s0 | s1 | s2)
+                            scatter_add<PLANES, B>(bx, by, s0, s1, s2, wox, woy, n, win, tkey, tplane, map);
                     }
                 }
             }
-        } else {
-            // spread cells: each lane its own bin columns and rows
-            for (int dx = 0; dx < nx; ++dx) {
-                const int bx = bxl + dx;
-                const float px = r * tri_clamped(xi, sxi, bx, bw);
-                if (px == 0.0f) continue;   // every contribution of this bin column is 0
-                for (int dy = 0; dy < ny; ++dy) {
-                    const int by = byl + dy;
-                    const float py = tri_clamped(yi, syi, by, bh);
-                    const unsigned long long c = (unsigned long long)fxp_rint_u64((px * py) * scale);
-                    if (c) scatter_add<PLANES>(bx, by, c, wox, woy, n, win, tkey, tplane, map);
-                }
-            }
         }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < kWin * kWin; k += blockDim.x) {
-        unsigned long long v = (unsigned long long)win[k] + ((unsigned long long)win[k + kWin * kWin] << 21);
-        if (PLANES == 3) v += (unsigned long long)win[k + 2 * kWin * kWin] << 42;
-        const int bx = wox + k / kWin, by = woy + k % kWin;
-        if (v && bx < m && by < n) atomicAdd(map + (size_t)bx * n + by, v);
-    }
-    for (int k = threadIdx.x; k < kTable; k += blockDim.x) {
-        const unsigned bin = tkey[k];
-        if (bin == kEmpty) continue;
-        unsigned long long v = (unsigned long long)tplane[k] + ((unsigned long long)tplane[k + kTable] << 21);
-        if (PLANES == 3) v += (unsigned long long)tplane[k + 2 * kTable] << 42;
-        if (v) atomicAdd(map + bin, v);
+        __syncthreads();
+        for (int k = threadIdx.x; k < kWin * kWin; k += blockDim.x) {
+            unsigned long long v = (unsigned long long)win[k] + ((unsigned long long)win[k + kWin * kWin] << B);
+            if (PLANES == 3) v += (unsigned long long)win[k + 2 * kWin * kWin] << 42;
+            const int bx = wox + k / kWin, by = woy + k % kWin;
+            if (v && bx < m && by < n) atomicAdd(map + (size_t)bx * n + by, v);
+        }
+        for (int k = threadIdx.x; k < kTable; k += blockDim.x) {
+            const unsigned bin = tkey[k];
+            if (bin == kEmpty) continue;
+            unsigned long long v = (unsigned long long)tplane[k] + ((unsigned long long)tplane[k + kTable] << B);
+            if (PLANES == 3) v += (unsigned long long)tplane[k + 2 * kTable] << 42;
+            if (v) atomicAdd(map + bin, v);
+        }
+        __syncthreads();   // the window is free for the next item
     }
 }
-template <int PLANES>
-__global__ void __launch_bounds__(kThreads) k_density_scatter(const __grid_constant__ ScatterP p) { density_scatter_body<PLANES>(p, blockIdx.x, gridDim.x); }
+template <int PLANES, int B>
+__global__ void __launch_bounds__(kThreads, 6) k_density_scatter(const __grid_constant__ ScatterP p) { density_scatter_body<PLANES, B>(p, blockIdx.x, gridDim.x); }
 
 
+// The window's forms by piece count and width.
+enum { SCATTER_2X21, SCATTER_2X23, SCATTER_3X21 };
+static int scatter_planes(int v) { return v == SCATTER_3X21 ? 3 : 2; }
+static void (*scatter_kernel(int v))(ScatterP) {
+    return v == SCATTER_2X21 ? k_density_scatter<2, 21> : (v == SCATTER_2X23 ? k_density_scatter<2, 23> : k_density_scatter<3, 21>);
+}
 size_t density_scatter_smem(int planes) { return sizeof(unsigned) * (planes * kWin * kWin + (planes + 1) * kTable); }
 
 // Scatter order: counting sort of the movable cells by sort tile.  Ranks within
@@ -665,26 +750,41 @@ __global__ void __launch_bounds__(kThreads) k_sort_count(int NM, const float2 *_
     }
 }
 
-// exclusive prefix sum of the tile counts (one block)
-__global__ void __launch_bounds__(1024) k_sort_scan(int ntiles, const int32_t *__restrict__ hist,
-                                                    int32_t *__restrict__ start) {
-    __shared__ int32_t part[1024];
+// Exclusive prefix sum of the tile counts, and the tiles' items (at most cap cells
+// each, a tile's items of equal size) in tile order; one block.
+__global__ void __launch_bounds__(1024) k_sort_scan(int ntiles, int nty, int m, int n, int cap,
+                                                    const int32_t *__restrict__ hist, int32_t *__restrict__ start,
+                                                    int4 *__restrict__ items, int32_t *__restrict__ n_items) {
+    __shared__ int2 part[1024];   // cells, items
     const int per = (ntiles + blockDim.x - 1) / blockDim.x;
     const int b = threadIdx.x * per, e = min(b + per, ntiles);
-    int32_t sum = 0;
-    for (int k = b; k < e; ++k) sum += hist[k];
+    int2 sum = make_int2(0, 0);
+    for (int k = b; k < e; ++k) {
+        const int h = hist[k];
+        sum.x += h;
+        sum.y += (h + cap - 1) / cap;
+    }
     part[threadIdx.x] = sum;
     __syncthreads();
     for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-        const int32_t v = (int)threadIdx.x >= off ? part[threadIdx.x - off] : 0;
+        const int2 v = (int)threadIdx.x >= off ? part[threadIdx.x - off] : make_int2(0, 0);
         __syncthreads();
-        part[threadIdx.x] += v;
+        part[threadIdx.x].x += v.x;
+        part[threadIdx.x].y += v.y;
         __syncthreads();
     }
-    int32_t run = threadIdx.x ? part[threadIdx.x - 1] : 0;
+    if (threadIdx.x == 0) *n_items = part[blockDim.x - 1].y;
+    int2 run = threadIdx.x ? part[threadIdx.x - 1] : make_int2(0, 0);
     for (int k = b; k < e; ++k) {
-        start[k] = run;
-        run += hist[k];
+        const int h = hist[k], cnt = (h + cap - 1) / cap;
+        start[k] = run.x;
+        const int wox = max(0, min((k / nty) * kSortTile - kSortPad, m - kWin));
+        const int woy = max(0, min((k % nty) * kSortTile - kSortPad, n - kWin));
+        const int each = cnt ? (h + cnt - 1) / cnt : 0;
+        for (int j = 0; j < cnt; ++j)
+            items[run.y + j] = make_int4(run.x + j * each, run.x + min((j + 1) * each, h), wox, woy);
+        run.x += h;
+        run.y += cnt;
     }
 }
 
@@ -696,7 +796,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_place(int NM, const int32_t *
                                                          const float *__restrict__ cw, const float *__restrict__ ch,
                                                          const float *__restrict__ ratio, int32_t *__restrict__ perm,
                                                          int32_t *__restrict__ pos, float4 *__restrict__ soff,
-                                                         float *__restrict__ sratio, int32_t *__restrict__ skey) {
+                                                         float *__restrict__ sratio) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NM; i += gridDim.x * blockDim.x) {
         const int k = key[i];
         const int p = start[k] + rank[i];
@@ -704,7 +804,6 @@ __global__ void __launch_bounds__(kThreads) k_sort_place(int NM, const int32_t *
         pos[i] = p;
         soff[p] = make_float4(offx[i], offy[i], cw[i], ch[i]);
         sratio[p] = ratio[i];
-        skey[p] = k;
     }
 }
 
@@ -712,11 +811,11 @@ int scatter_tiles(int m, int n) { return ((m + kSortTile - 1) / kSortTile) * ((n
 
 static cudaError_t packed_prepare();
 cudaError_t place_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(k_density_scatter<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)density_scatter_smem(2));
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_density_scatter<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)density_scatter_smem(3));
+    cudaError_t e = cudaSuccess;
+    for (int v : {SCATTER_2X21, SCATTER_2X23, SCATTER_3X21})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(scatter_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)density_scatter_smem(scatter_planes(v)));
     if (e != cudaSuccess) return e;
     return packed_prepare();
 }
@@ -1394,26 +1493,41 @@ void launch_wl_gather(Ctx &c) {
     k_wl_gather<<<g, kThreads, 0, c.stream>>>(p);
 }
 
-// Blocks of the scatter.  Alone, a context spreads its cells over up to 608
-// blocks (four per SM); a batch autotunes the cells per block, since with many
-// instances on the GPU at once fewer, fuller blocks flush fewer windows (see
-// erp_batch_create).  Never more than kMaxCellsPerBlock cells per block (the
-// window's 21-bit pieces rely on it); the grid decides no bit of the map.
-static int scatter_params(Ctx &c, ScatterP &p) {
-    const int floor_g = (c.NM + kMaxCellsPerBlock - 1) / kMaxCellsPerBlock;
-    const int g = c.scatter_cells > 0 ? std::max((c.NM + c.scatter_cells - 1) / c.scatter_cells, std::max(floor_g, 1))
-                                      : std::max(grid_for(c.NM, 152 * 4), floor_g);
-    const int nty = (c.n + kSortTile - 1) / kSortTile;
-    p = ScatterP{c.NM, c.perm, c.xy, c.soff, c.sratio, c.skey, nty, c.m, c.n, c.bin_w, c.bin_h, c.inv_bw, c.inv_bh,
+// Cells per item of the scatter (a multiple of 32).  Alone, a context spreads its
+// cells over about 608 blocks (four per SM) of at least 256; a batch autotunes the
+// number, since with many instances on the GPU at once fewer, fuller blocks flush
+// fewer windows (see erp_batch_create).  Never more than kMaxCellsPerBlock (the
+// window's pieces rely on it); the items decide no bit of the map.
+static int scatter_cap(const Ctx &c) {
+    const int cells = c.scatter_cells > 0 ? c.scatter_cells : (c.NM + 152 * 4 - 1) / (152 * 4);
+    const int least = c.scatter_cells > 0 ? 32 : 256;
+    return std::min((std::max(cells, least) + 31) & ~31, kMaxCellsPerBlock);
+}
+
+// Items there can be: every tile with cells may hold one that is not full.
+static int scatter_items(const Ctx &c, int cap) { return std::min(scatter_tiles(c.m, c.n), c.NM) + (c.NM + cap - 1) / cap; }
+int scatter_items_max(int NM, int m, int n) { return std::min(scatter_tiles(m, n), NM) + (NM + 31) / 32; }
+
+static int scatter_params(Ctx &c, ScatterP &p, int &variant) {
+    const int cap = scatter_cap(c);
+    p = ScatterP{c.perm, c.xy, c.soff, c.sratio, c.items, c.n_items, c.NM >= kFollowCells, c.m, c.n, c.bin_w, c.bin_h, c.inv_bw, c.inv_bh,
                  c.fixed_scale, c.dmap, c.st};
-    return g;
+    variant = c.scatter_bits <= 42 ? SCATTER_2X21 : (c.scatter_bits <= 46 && cap <= 512 ? SCATTER_2X23 : SCATTER_3X21);
+    return std::max(scatter_items(c, cap), 1);
 }
 
 void launch_density_scatter(Ctx &c) {
     ScatterP p;
-    const int g = scatter_params(c, p);
-    auto kern = c.scatter_planes == 2 ? k_density_scatter<2> : k_density_scatter<3>;
-    kern<<<g, kThreads, density_scatter_smem(c.scatter_planes), c.stream>>>(p);
+    int v;
+    const int g = scatter_params(c, p, v);
+    scatter_kernel(v)<<<g, kThreads, density_scatter_smem(scatter_planes(v)), c.stream>>>(p);
+}
+
+// The items of the current order again, after scatter_cells changed.
+void launch_scatter_items(Ctx &c, cudaStream_t s) {
+    if (c.NM <= 0) return;
+    k_sort_scan<<<1, 1024, 0, s>>>(scatter_tiles(c.m, c.n), (c.n + kSortTile - 1) / kSortTile, c.m, c.n, scatter_cap(c),
+                                   c.sort_hist, c.sort_start, c.items, c.n_items);
 }
 
 void launch_scatter_order(Ctx &c, cudaStream_t s) {
@@ -1424,10 +1538,9 @@ void launch_scatter_order(Ctx &c, cudaStream_t s) {
     k_sort_count<<<(c.NM + 4 * kThreads - 1) / (4 * kThreads), kThreads, sizeof(int32_t) * ntiles, s>>>(
         c.NM, c.xy, c.offx, c.offy, c.inv_bw, c.inv_bh, c.m, c.n, nty, ntiles, c.sort_key, c.sort_rank,
         c.sort_hist);
-    k_sort_scan<<<1, 1024, 0, s>>>(ntiles, c.sort_hist, c.sort_start);
+    launch_scatter_items(c, s);
     k_sort_place<<<grid_for(c.NM), kThreads, 0, s>>>(c.NM, c.sort_key, c.sort_rank, c.sort_start, c.offx, c.offy,
-                                                     c.cw, c.ch, c.ratio, c.perm, c.pos, c.soff, c.sratio,
-                                                     c.skey);
+                                                     c.cw, c.ch, c.ratio, c.perm, c.pos, c.soff, c.sratio);
 }
 
 void launch_initial_density(Ctx &c, const float *, const float *, const float *, const float *) {
@@ -1640,12 +1753,19 @@ void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &a
         plan_stage<GatherP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, GatherP &p) { return gather_params(c, p); });
         break;
     case PK_SCATTER:
-        for (int planes = 2; planes <= 3; ++planes) {
+        for (int v : {SCATTER_2X21, SCATTER_2X23, SCATTER_3X21}) {
             std::vector<Ctx *> sub;
-            for (Ctx *c : xs)
-                if (c->scatter_planes == planes) sub.push_back(c);
-            plan_stage<ScatterP>(k, planes, sub, ar, out, kThreads, density_scatter_smem(planes),
-                                 [](Ctx &c, ScatterP &p) { return scatter_params(c, p); });
+            for (Ctx *c : xs) {
+                ScatterP p;
+                int cv;
+                scatter_params(*c, p, cv);
+                if (cv == v) sub.push_back(c);
+            }
+            plan_stage<ScatterP>(k, v, sub, ar, out, kThreads, density_scatter_smem(scatter_planes(v)),
+                                 [](Ctx &c, ScatterP &p) {
+                                     int cv;
+                                     return scatter_params(c, p, cv);
+                                 });
         }
         break;
     case PK_FORCE:
@@ -1662,12 +1782,18 @@ void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &a
     }
 }
 
+static void (*packed_scatter_kernel(int v))(Packed<ScatterP>) {
+    return v == SCATTER_2X21 ? k_packed<ScatterP, density_scatter_body<2, 21>, kThreads, 4>
+                             : (v == SCATTER_2X23 ? k_packed<ScatterP, density_scatter_body<2, 23>, kThreads, 4>
+                                                  : k_packed<ScatterP, density_scatter_body<3, 21>, kThreads, 4>);
+}
 static cudaError_t packed_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(k_packed<ScatterP, density_scatter_body<2>, kThreads, 4>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)density_scatter_smem(2));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_packed<ScatterP, density_scatter_body<3>, kThreads, 4>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)density_scatter_smem(3));
+    cudaError_t e = cudaSuccess;
+    for (int v : {SCATTER_2X21, SCATTER_2X23, SCATTER_3X21})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(packed_scatter_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)density_scatter_smem(scatter_planes(v)));
+    return e;
 }
 
 bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaStream_t s) {
@@ -1679,12 +1805,7 @@ bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaSt
         k_packed<GatherP, wl_gather_body, kThreads, 4><<<l.blocks, l.threads, 0, s>>>(packed_args<GatherP>(l, dev));
         return true;
     case PK_SCATTER:
-        if (l.variant == 2)
-            k_packed<ScatterP, density_scatter_body<2>, kThreads, 4><<<l.blocks, l.threads, l.smem, s>>>(
-                packed_args<ScatterP>(l, dev));
-        else
-            k_packed<ScatterP, density_scatter_body<3>, kThreads, 4><<<l.blocks, l.threads, l.smem, s>>>(
-                packed_args<ScatterP>(l, dev));
+        packed_scatter_kernel(l.variant)<<<l.blocks, l.threads, l.smem, s>>>(packed_args<ScatterP>(l, dev));
         return true;
     case PK_FORCE:
         k_packed<ForceP, force_body, kThreads, 4><<<l.blocks, l.threads, 0, s>>>(packed_args<ForceP>(l, dev));
