@@ -273,11 +273,17 @@ static SpectralArgs spectral_args(Ctx &c, bool zero_map, bool store_rho, bool wa
     a.rho_out = store_rho ? c.rho : nullptr;
     a.fx = c.fx;
     a.fy = c.fy;
+    a.field_stride = c.field_pairs ? 2 : 1;
     a.psi = want_psi ? c.psi : nullptr;
     a.partials = step ? c.part_ovf : c.partials;
     a.st = c.st;
     a.step = step;
     return a;
+}
+
+void set_field_pairs(Ctx &c, bool pairs) {
+    c.field_pairs = pairs && !c.gemm;
+    c.fy = c.fx + (c.field_pairs ? 1 : (size_t)c.m * c.n);
 }
 
 int overflow_blocks(const Ctx &c) {
@@ -498,8 +504,9 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     ap.add(&c.sort_hist, scatter_tiles(c.m, c.n));
     ap.add(&c.sort_start, scatter_tiles(c.m, c.n));
     ap.add(&c.dmap, mn);
-    float **maps[] = {&c.initial, &c.rho, &c.t1, &c.tx, &c.ty, &c.tp, &c.fx, &c.fy, &c.psi};
+    float **maps[] = {&c.initial, &c.rho, &c.t1, &c.tx, &c.ty, &c.tp, &c.psi};
     for (float **a : maps) ap.add(a, mn);
+    ap.add(&c.fx, 2 * mn);
     ap.add(&c.partials, kMaxPartials);
     ap.add(&c.part_wl, kMaxPartials);
     ap.add(&c.part_ovf, kMaxRowBlocks);
@@ -526,6 +533,7 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
                                 c.err);
         if (!c.gemm) return ERP_ECUDA;
     }
+    set_field_pairs(c, NM >= kFieldPairCells);
     // --- uploads ---
     CK(upload(c.x, hx.data(), sizeof(float) * N, c.stream));
     CK(upload(c.y, hy.data(), sizeof(float) * N, c.stream));
@@ -552,6 +560,7 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     CK(upload(c.cell_slots, hcell_slots.data(), sizeof(int32_t) * hcell_slots.size(), c.stream));
     CK(cudaMemsetAsync(c.dmap, 0, sizeof(unsigned long long) * mn, c.stream));
     for (float **a : maps) CK(cudaMemsetAsync(*a, 0, sizeof(float) * mn, c.stream));
+    CK(cudaMemsetAsync(c.fx, 0, sizeof(float) * 2 * mn, c.stream));
     // scheduler / optimiser state (src/scheduler.rs:52-66, src/nesterov.rs:15-24)
     DevState h;
     memset(&h, 0, sizeof h);
@@ -967,8 +976,20 @@ extern "C" erp_status erp_get_array(erp_ctx *ctx, erp_array which, void *dst, si
     case ERP_ARR_DENSITY_I64: src = c.dmap; need = sizeof(int64_t) * mn; break;
     case ERP_ARR_DENSITY: src = c.rho; need = sizeof(float) * mn; break;
     case ERP_ARR_INITIAL: src = c.initial; need = sizeof(float) * mn; break;
-    case ERP_ARR_FIELD_X: src = c.fx; need = sizeof(float) * mn; break;
-    case ERP_ARR_FIELD_Y: src = c.fy; need = sizeof(float) * mn; break;
+    case ERP_ARR_FIELD_X:
+    case ERP_ARR_FIELD_Y:
+        src = which == ERP_ARR_FIELD_X ? c.fx : c.fy;
+        need = sizeof(float) * mn;
+        if (c.field_pairs) {   // interleaved on the device
+            if (bytes < need) { c.err = "destination too small"; return ERP_EINVAL; }
+            std::vector<float2> f(mn);
+            CK(cudaMemcpyAsync(f.data(), c.fx, sizeof(float2) * mn, cudaMemcpyDeviceToHost, c.stream));
+            CK(cudaStreamSynchronize(c.stream));
+            float *o = (float *)dst;
+            for (size_t k = 0; k < mn; ++k) o[k] = which == ERP_ARR_FIELD_X ? f[k].x : f[k].y;
+            return ERP_OK;
+        }
+        break;
     case ERP_ARR_POTENTIAL: src = c.psi; need = sizeof(float) * mn; break;
     case ERP_ARR_PREV_X: src = c.prev_x; need = sizeof(float) * c.N; break;
     case ERP_ARR_PREV_Y: src = c.prev_y; need = sizeof(float) * c.N; break;
@@ -1364,6 +1385,9 @@ extern "C" erp_status erp_batch_create(const erp_design *designs, const erp_para
         if (b->packed)
             for (auto *x : b->ctx) b->packed_instances += packable(x->c) ? 1 : 0;
         if (b->packed_instances < kPackMin) b->packed_instances = 0;
+        if (b->packed_instances)   // together they have the cells for which interleaved fields pay
+            for (auto *x : b->ctx)
+                if (packable(x->c)) set_field_pairs(x->c, true);
     }
     if (s != ERP_OK) {
         erp_batch_destroy(b);
@@ -1912,7 +1936,7 @@ extern "C" erp_status erp_estimate_footprint(const erp_design *d, const erp_para
     auto al = [](int64_t v) { return (v + 511) & ~int64_t(511); };   // allocation granularity
     int64_t b = 16 * al(4 * (N + 4));
     b += al(4 * P) + 2 * al(8 * P) + al(4 * (E + 1)) + al(4 * E) + al(4 * (NM + 1)) + al(4 * movable_pins);
-    b += al(8 * mn) + 9 * al(4 * mn) + 2 * al(8 * (int64_t)kMaxPartials) +
+    b += al(8 * mn) + 7 * al(4 * mn) + al(8 * mn) + 2 * al(8 * (int64_t)kMaxPartials) +
          al(8 * (int64_t)kMaxRowBlocks) + al(sizeof(DevState));
     b += 4 * al(4 * (int64_t)NM) + al(16 * (int64_t)scatter_items_max((int)NM, m, n)) + 512 + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)scatter_tiles(m, n));   // scatter order
     b += al(4 * (NM + 4)) + al(8 * (NM + 4));   // its inverse, the density gradient in that order

@@ -125,7 +125,9 @@ struct Ctx {
     int32_t *h_net_of_internal;// [E]
     // --- maps [m*n] ---
     unsigned long long *dmap;  // int64 fixed-point movable density
-    float *initial, *rho, *t1, *tx, *ty, *tp, *fx, *fy, *psi;
+    float *initial, *rho, *t1, *tx, *ty, *tp, *psi;
+    float *fx, *fy;            // two maps in one array [2 m*n], or interleaved
+    bool field_pairs;          // interleaved: (field_x, field_y) per bin, fy = fx + 1 (see set_field_pairs)
     float2 *tw_m, *tw_n, *ek_m, *ek_n;   // FFT twiddles and DCT post-twiddles
     float *wu, *wv;            // frequency vectors [m], [n]
     bool map_dirty;
@@ -163,6 +165,10 @@ void launch_initial_density(Ctx &c, const float *hx, const float *hy, const floa
                             const float *hh);               // setup, on device
 void launch_density_scatter(Ctx &c);
 void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step);
+// The layout of the two fields between the solve and the force (before a step or
+// a stage uses them): interleaved, or (always with the tensor-core solve) two maps.
+constexpr int kFieldPairCells = 131072;   // alone, designs of this many movable cells interleave (see k_force)
+void set_field_pairs(Ctx &c, bool pairs);
 int overflow_blocks(const Ctx &c);   // block sums the overflow has in this context's step
 void launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
 void launch_scatter_items(Ctx &c, cudaStream_t s);   // its work items again, after scatter_cells changed
@@ -257,6 +263,7 @@ struct SpectralArgs {
     bool zero_map = false;
     float *rho_out = nullptr;
     float *fx = nullptr, *fy = nullptr, *psi = nullptr;
+    int field_stride = 1;                   // elements between neighbouring bins in fx and fy: 2 when interleaved
     double *partials = nullptr;
     DevState *st = nullptr;
     bool step = false;                      // part of a whole step: leave the overflow's block sums in partials

@@ -871,7 +871,13 @@ __device__ __forceinline__ float tri_raw(float x, float s, int k, float bs) {
     return fminf(x + s, bin_xl + bs) - fmaxf(x, bin_xl);
 }
 
-// compute_electric_force (src/eforce.rs:15-91)
+// compute_electric_force (src/eforce.rs:15-91).  With many cells the pass is bound by
+// its gathers (L1 wavefronts and L2 latency): the FFT solve then interleaves the two
+// fields, one 8-byte load per bin, and a cell's loads are unrolled.  1M cells over
+// 1024^2 bins: 17.2 -> 14.7 us with a fresh order, 28 -> 19 us in steps that move the
+// cells by tens of bins, against 1.4 us more in the solve's last pass; 550,000 cells in
+// 32 packed instances 17.3 -> 14.3 us.  One small design has too few warps for that to
+// matter and keeps two maps (20,000 cells: 4.4 against 5.2 us).
 struct ForceP {
     int NM;
     const int32_t * perm;
@@ -889,7 +895,7 @@ struct ForceP {
     float bh;
     float inv_bw;
     float inv_bh;
-    const float * fx;
+    const float * fx;   // PAIRS: (field_x, field_y) interleaved
     const float * fy;
     float2 * dgp;
     const int32_t * pos;
@@ -899,6 +905,7 @@ struct ForceP {
     double * partials;
     DevState * st;
 };
+template <bool PAIRS>
 __device__ __forceinline__ void force_body(const ForceP &p, int bid, int nblk) {
     int NM = p.NM;
     const int32_t *__restrict__ perm = p.perm;
@@ -927,21 +934,50 @@ __device__ __forceinline__ void force_body(const ForceP &p, int bid, int nblk) {
     DevState * st = p.st;
     __shared__ double shr[kThreads / 32];
     if (st->done) return;
-    // the field gathered over cell i's bins (src/eforce.rs)
+    auto field = [&](int at) -> float2 {
+        if (PAIRS) return __ldg(reinterpret_cast<const float2 *>(fx) + at);
+        return make_float2(__ldg(fx + at), __ldg(fy + at));
+    };
+    // The field gathered over a cell's bins (src/eforce.rs:48-83).
     auto force = [&](float nx, float ny, float sx, float sy, float r) -> float2 {
         const int xl = force_bin_lo((nx - 0.0f) * inv_bw, m);
         const int xh = force_bin_hi((nx + sx - 0.0f) * inv_bw, m);
         const int yl = force_bin_lo((ny - 0.0f) * inv_bh, n);
         const int yh = force_bin_hi((ny + sy - 0.0f) * inv_bh, n);
         float gx = 0.0f, gy = 0.0f;
+        const int cx = xh - xl, cy = yh - yl;
+        if (PAIRS && cx <= 3 && cy <= 3) {
+            // cells of less than two bins: all loads issued before the first is used,
+            // the products added in the loops' order (same bits)
+            const int at = xl * n + yl;   // at most 2^24 bins
+            float px[3], py[3];
+            float2 v[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                v[k] = k / 3 < cx && k % 3 < cy ? field(at + k / 3 * n + k % 3) : make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                px[k] = tri_raw(nx, sx, xl + k, bw);
+                py[k] = tri_raw(ny, sy, yl + k, bh);
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const float area = px[k / 3] * py[k % 3];
+                if (k / 3 < cx && k % 3 < cy) {
+                    gx += area * v[k].x;
+                    gy += area * v[k].y;
+                }
+            }
+            return make_float2(-gx * r, -gy * r);
+        }
         for (int k = xl; k < xh; ++k) {
             const float px = tri_raw(nx, sx, k, bw);
-            const float *rx = fx + (size_t)k * n, *ry = fy + (size_t)k * n;
             for (int hh = yl; hh < yh; ++hh) {
                 const float py = tri_raw(ny, sy, hh, bh);
                 const float area = px * py;
-                gx += area * __ldg(rx + hh);
-                gy += area * __ldg(ry + hh);
+                const float2 v = field(k * n + hh);
+                gx += area * v.x;
+                gy += area * v.y;
             }
         }
         return make_float2(-gx * r, -gy * r);
@@ -987,7 +1023,8 @@ __device__ __forceinline__ void force_body(const ForceP &p, int bid, int nblk) {
         dgp[p] = force(q.x + o.x, q.y + o.y, o.z, o.w, sratio[p]);
     }
 }
-__global__ void __launch_bounds__(kThreads) k_force(const __grid_constant__ ForceP p) { force_body(p, blockIdx.x, gridDim.x); }
+template <bool PAIRS>
+__global__ void __launch_bounds__(kThreads) k_force(const __grid_constant__ ForceP p) { force_body<PAIRS>(p, blockIdx.x, gridDim.x); }
 
 
 // energy = sum psi * rho (src/epotential.rs:344-346), double-float sums
@@ -1594,7 +1631,7 @@ static int force_params(Ctx &c, int rescale, ForceP &p) {
 void launch_force(Ctx &c, int rescale) {
     ForceP p;
     const int g = force_params(c, rescale, p);
-    k_force<<<g, kThreads, 0, c.stream>>>(p);
+    (c.field_pairs ? k_force<true> : k_force<false>)<<<g, kThreads, 0, c.stream>>>(p);
 }
 
 void launch_energy(Ctx &c) {
@@ -1645,7 +1682,7 @@ cudaError_t place_occupancy() {
     int dev = 0, sms = 0, a = 0, b = 0, d = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_force, kThreads, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_force<true>, kThreads, 0);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_nesterov_grad, kThreads, 0);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_nesterov_update, kThreads, 0);
     if (e != cudaSuccess) return e;
@@ -1769,7 +1806,12 @@ void packed_place_stage(PackKind k, const std::vector<Ctx *> &xs, PackedArena &a
         }
         break;
     case PK_FORCE:
-        plan_stage<ForceP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, ForceP &p) { return force_params(c, 1, p); });
+        for (int pairs = 0; pairs < 2; ++pairs) {
+            std::vector<Ctx *> sub;
+            for (Ctx *c : xs)
+                if ((int)c->field_pairs == pairs) sub.push_back(c);
+            plan_stage<ForceP>(k, pairs, sub, ar, out, kThreads, 0, [](Ctx &c, ForceP &p) { return force_params(c, 1, p); });
+        }
         break;
     case PK_GRAD:
         plan_stage<GradP>(k, 0, xs, ar, out, kThreads, 0, [](Ctx &c, GradP &p) { return grad_params(c, -1, true, p); });
@@ -1808,7 +1850,8 @@ bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaSt
         packed_scatter_kernel(l.variant)<<<l.blocks, l.threads, l.smem, s>>>(packed_args<ScatterP>(l, dev));
         return true;
     case PK_FORCE:
-        k_packed<ForceP, force_body, kThreads, 4><<<l.blocks, l.threads, 0, s>>>(packed_args<ForceP>(l, dev));
+        (l.variant ? k_packed<ForceP, force_body<true>, kThreads, 4>
+                   : k_packed<ForceP, force_body<false>, kThreads, 4>)<<<l.blocks, l.threads, 0, s>>>(packed_args<ForceP>(l, dev));
         return true;
     case PK_GRAD:
         k_packed<GradP, nesterov_grad_body, kThreads, 3><<<l.blocks, l.threads, 0, s>>>(packed_args<GradP>(l, dev));

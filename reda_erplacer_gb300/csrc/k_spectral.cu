@@ -252,7 +252,7 @@ template <int PAIRS>
 __global__ void __launch_bounds__(kThreads) k_rows_inv_r2(
     int m, int n, int logn, const float2 *__restrict__ tw_g, const float2 *__restrict__ ek_n,
     const float *__restrict__ tx, const float *__restrict__ ty, const float *__restrict__ tp,
-    float *__restrict__ fx, float *__restrict__ fy, float *__restrict__ psi,
+    float *__restrict__ fx, float *__restrict__ fy, float *__restrict__ psi, int field_stride,
     const DevState *__restrict__ st) {
     if (st && st->done) return;
     extern __shared__ __align__(16) float2 sm[];
@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(kThreads) k_rows_inv_r2(
         // kind 0: field_x = IDCT_n(tx); kind 1: field_y = IDXST_n(ty); kind 2: psi = IDCT_n(tp)
         const float *in = kind == 0 ? tx : (kind == 1 ? ty : tp);
         float *out = kind == 0 ? fx : (kind == 1 ? fy : psi);
+        const size_t fs = kind == 2 ? 1 : field_stride;
         const bool sine = kind == 1;
         for (int idx = threadIdx.x; idx < PAIRS * n; idx += blockDim.x) {
             const int p = idx >> logn, i = idx & (n - 1);
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(kThreads) k_rows_inv_r2(
             float va = w.x, vb = w.y;
             if (sine && (i & 1)) { va = -va; vb = -vb; }
             const int r = row0 + 2 * p;
-            out[(size_t)r * n + i] = va;
-            out[(size_t)(r + 1) * n + i] = vb;
+            out[((size_t)r * n + i) * fs] = va;
+            out[((size_t)(r + 1) * n + i) * fs] = vb;
         }
         __syncthreads();
     }
@@ -610,6 +611,7 @@ struct RowsInvP {
     float * fy;
     float * psi;
     int pairs;   // 1: the outputs start on 8-byte boundaries (a caller's buffer may not)
+    int field_stride;   // elements between neighbouring bins of a field: 2 when interleaved
     const DevState * st;
 };
 template <int N, int P>
@@ -625,7 +627,8 @@ __device__ __forceinline__ void rows_inv_body(const RowsInvP &a, int bid, int nb
     const int pair = fields ? task >> 1 : task;   // rows at positions 2 pair and 2 pair + 1
     const float2 *in = reinterpret_cast<const float2 *>(kind == 0 ? a.tx : (kind == 1 ? a.ty : a.tp)) + (size_t)pair * N;
     float *out = kind == 0 ? a.fx : (kind == 1 ? a.fy : a.psi);
-    float *oa = out + (size_t)makhoul_elem(2 * pair, a.m) * N, *ob = out + (size_t)makhoul_elem(2 * pair + 1, a.m) * N;
+    const int fs = kind == 2 ? 1 : a.field_stride;
+    float *oa = out + (size_t)makhoul_elem(2 * pair, a.m) * N * fs, *ob = out + (size_t)makhoul_elem(2 * pair + 1, a.m) * N * fs;
     const bool sine = kind == 1;
     float2 v[F::R1], w1[F::R1], xn[F::R1], ek[F::R1];
 #pragma unroll
@@ -655,14 +658,14 @@ __device__ __forceinline__ void rows_inv_body(const RowsInvP &a, int bid, int nb
         const int s = t + j * F::T;   // elements 2 s and 2 s + 1
         float2 z0 = sm[s * P + p], z1 = sm[(N - 1 - s) * P + p];
         if (sine) z1 = make_float2(-z1.x, -z1.y);
-        if (a.pairs) {
+        if (a.pairs && fs == 1) {
             reinterpret_cast<float2 *>(oa)[s] = make_float2(z0.x, z1.x);
             reinterpret_cast<float2 *>(ob)[s] = make_float2(z0.y, z1.y);
         } else {
-            oa[2 * s] = z0.x;
-            oa[2 * s + 1] = z1.x;
-            ob[2 * s] = z0.y;
-            ob[2 * s + 1] = z1.y;
+            oa[2 * s * fs] = z0.x;
+            oa[(2 * s + 1) * fs] = z1.x;
+            ob[2 * s * fs] = z0.y;
+            ob[(2 * s + 1) * fs] = z1.y;
         }
     }
 }
@@ -865,7 +868,7 @@ struct LaunchRowsInv {
         const uintptr_t at = reinterpret_cast<uintptr_t>(a.fx) | reinterpret_cast<uintptr_t>(a.fy) |
                              reinterpret_cast<uintptr_t>(a.psi);
         return RowsInvP{p.m,  p.tw_n, p.ek_n, p.tx, p.ty, a.psi ? p.tp : nullptr, a.fx, a.fy, a.psi, (at & 7) == 0,
-                        a.st};
+                        a.field_stride, a.st};
     }
     static int blocks(int m, int P, bool psi) { return m / P + (psi ? m / (2 * P) : 0); }
     template <int N, int P>
@@ -939,7 +942,7 @@ void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a) {
         pair_dispatch<PASS_ROWS_INV>(n, p.seqs, LaunchRowsInv{p, a});
     } else {
         k_rows_inv_r2<kRowPairs><<<rb, kThreads, rows_smem(n, kRowPairs), p.stream>>>(
-            m, n, p.logn, p.tw_n, p.ek_n, p.tx, p.ty, tp, a.fx, a.fy, a.psi, a.st);
+            m, n, p.logn, p.tw_n, p.ek_n, p.tx, p.ty, tp, a.fx, a.fy, a.psi, a.field_stride, a.st);
     }
 }
 
