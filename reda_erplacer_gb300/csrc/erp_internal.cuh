@@ -183,8 +183,9 @@ void launch_energy(Ctx &c);
 // optimiser + scheduler (src/nesterov.rs, src/scheduler.rs)
 void launch_nesterov(Ctx &c, int iter_arg, bool step);     // iter_arg < 0: read DevState.iteration
 void launch_scheduler(Ctx &c, int use_args, float hpwl, float overflow);
-// One whole Placement::step on the context's stream (the graph's content).
-void enqueue_step_kernels(Ctx &c);
+// One whole Placement::step on the context's stream (the graph's content); with a
+// second stream and two events, under capture, in two branches up to the force.
+void enqueue_step_kernels(Ctx &c, cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 // Gather the retire flags of several contexts into out[i] (device pointers).
 void launch_gather_done(DevState *const *states, int count, int32_t *out, cudaStream_t s);
 
@@ -287,7 +288,7 @@ cudaError_t spectral_prepare();
 // tensor-core form of the spectral solve (k_dctgemm.cu): kind 0 TF32, 1 BF16x3
 DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cudaStream_t stream,
                             std::string &err);
-cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status);
+cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status, cudaStream_t s);
 void dctgemm_destroy(DctGemmPlan *P);
 cudaError_t place_prepare();   // opt the density scatter into its dynamic shared memory
 

@@ -495,19 +495,18 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
 }
 
 template <int KIND, int BN>
-static cudaError_t launch_gemm(const DctGemmPlan &P, const GemmMaps &maps, const GemmEpi &epi, int M, int N,
-                               int K, int Z) {
+static cudaError_t launch_gemm(const GemmMaps &maps, const GemmEpi &epi, int M, int N, int K, int Z, cudaStream_t s) {
     dim3 grid(N / BN, M / kTile, Z);
-    k_gemm_nt<KIND, BN><<<grid, 128, GemmCfg<KIND, BN>::kSmem, P.stream>>>(maps, epi, K);
+    k_gemm_nt<KIND, BN><<<grid, 128, GemmCfg<KIND, BN>::kSmem, s>>>(maps, epi, K);
     return cudaGetLastError();
 }
 
 static cudaError_t run_gemm(const DctGemmPlan &P, const GemmMaps &maps, const GemmEpi &epi, int M, int N, int K,
-                            int Z, int bn) {
+                            int Z, int bn, cudaStream_t s) {
     if (bn == 64)
-        return P.kind == 0 ? launch_gemm<0, 64>(P, maps, epi, M, N, K, Z) : launch_gemm<1, 64>(P, maps, epi, M, N, K, Z);
-    return P.kind == 0 ? launch_gemm<0, 128>(P, maps, epi, M, N, K, Z)
-                       : launch_gemm<1, 128>(P, maps, epi, M, N, K, Z);
+        return P.kind == 0 ? launch_gemm<0, 64>(maps, epi, M, N, K, Z, s) : launch_gemm<1, 64>(maps, epi, M, N, K, Z, s);
+    return P.kind == 0 ? launch_gemm<0, 128>(maps, epi, M, N, K, Z, s)
+                       : launch_gemm<1, 128>(maps, epi, M, N, K, Z, s);
 }
 
 // fx, fy (, psi) = Poisson solve of rho: four contraction launches (+ the split
@@ -517,14 +516,14 @@ static cudaError_t run_gemm(const DctGemmPlan &P, const GemmMaps &maps, const Ge
 // status: where the contractions report a bounded wait that ran out; nullptr
 // uses the plan's own word and its pinned mirror (a placement context passes
 // its DevState status, read by the host with the rest of the state).
-cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status) {
+cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status, cudaStream_t s) {
     if (!status && *(volatile int *)P.h_status) return cudaErrorTimeout;
     const int m = P.m, n = P.n, nk = psi ? 3 : 2;
     const size_t mn = (size_t)m * n;
     const bool split = P.kind == 1;
     cudaError_t e = cudaSuccess;
     if (split) {
-        k_split_bf16<<<152 * 8, 256, 0, P.stream>>>(mn, rho, (__nv_bfloat16 *)P.rho2.p[0],
+        k_split_bf16<<<152 * 8, 256, 0, s>>>(mn, rho, (__nv_bfloat16 *)P.rho2.p[0],
                                                    (__nv_bfloat16 *)P.rho2.p[1]);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else if (rho != P.rho_cached) {
@@ -539,23 +538,23 @@ cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy
     // G1: Z = rho C_n^T, stored transposed [n][m]
     ep.mode = 0; ep.transpose = 1; ep.alpha = 1.0f; ep.ldc = m;
     ep.out[0][0] = P.Zt.p[0]; ep.out[0][1] = P.Zt.p[1];
-    if ((e = run_gemm(P, P.g1, ep, m, n, n, 1, 64)) != cudaSuccess) return e;
+    if ((e = run_gemm(P, P.g1, ep, m, n, n, 1, 64, s)) != cudaSuccess) return e;
     // G2: A = (4/mn) C_m Z, written as the weighted spectra [m][n]
     ep.mode = 1; ep.transpose = 0; ep.alpha = (float)(4.0 / ((double)m * (double)n)); ep.ldc = n;
     ep.nplanes = nk; ep.wu = P.wu; ep.wv = P.wv;
     for (int k = 0; k < 3; ++k) { ep.out[k][0] = P.Aw[k].p[0]; ep.out[k][1] = P.Aw[k].p[1]; }
-    if ((e = run_gemm(P, P.g2, ep, m, n, m, 1, 64)) != cudaSuccess) return e;
+    if ((e = run_gemm(P, P.g2, ep, m, n, m, 1, 64, s)) != cudaSuccess) return e;
     // G3: Z_k = Aw_k (D_n | S_n | D_n)^T, stored transposed [n][m]
     ep.mode = 0; ep.transpose = 1; ep.alpha = 1.0f; ep.ldc = m; ep.nplanes = 0;
     for (int k = 0; k < 3; ++k) { ep.out[k][0] = P.Zkt[k].p[0]; ep.out[k][1] = P.Zkt[k].p[1]; }
-    if ((e = run_gemm(P, P.g3, ep, m, n, n, nk, 128)) != cudaSuccess) return e;
+    if ((e = run_gemm(P, P.g3, ep, m, n, n, nk, 128, s)) != cudaSuccess) return e;
     // G4: field_x = S_m Z_x, field_y = D_m Z_y, psi = D_m Z_p, fp32 [m][n]
     ep.split = 0; ep.transpose = 0; ep.ldc = n;
     float *outs[3] = {fx, fy, psi};
     for (int k = 0; k < 3; ++k) { ep.out[k][0] = outs[k]; ep.out[k][1] = nullptr; }
-    if ((e = run_gemm(P, P.g4, ep, m, n, m, nk, 128)) != cudaSuccess) return e;
+    if ((e = run_gemm(P, P.g4, ep, m, n, m, nk, 128, s)) != cudaSuccess) return e;
     if (status) return cudaSuccess;
-    return cudaMemcpyAsync(P.h_status, P.status, sizeof(int), cudaMemcpyDeviceToHost, P.stream);
+    return cudaMemcpyAsync(P.h_status, P.status, sizeof(int), cudaMemcpyDeviceToHost, s);
 }
 
 }  // namespace erp
