@@ -294,8 +294,10 @@ int overflow_blocks(const Ctx &c) {
 void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool step) {
     const SpectralArgs a = spectral_args(c, zero_map, store_rho, want_psi, step);
     if (c.gemm) {   // tensor-core precisions: rho, then the contractions (rho_out is c.rho itself)
-        launch_map_rho(a, (size_t)c.m * c.n, c.rho, c.stream);
-        dctgemm_solve(*c.gemm, c.rho, c.fx, c.fy, a.psi, &c.st->status, c.stream);
+        void *hi, *lo;
+        const bool parts = dctgemm_input_parts(*c.gemm, &hi, &lo);
+        launch_map_rho(a, (size_t)c.m * c.n, c.rho, parts ? hi : nullptr, parts ? lo : nullptr, c.stream);
+        dctgemm_solve(*c.gemm, parts ? nullptr : c.rho, c.fx, c.fy, a.psi, &c.st->status, c.stream);
         return;
     }
     launch_spectral_plan(plan_of(c), a);

@@ -283,11 +283,13 @@ void packed_spectral_stage(PackKind k, const std::vector<SpectralJob> &v, Packed
                            std::vector<PackedLaunch> &out);
 bool packed_spectral_launch(const PackedLaunch &l, const unsigned char *dev, cudaStream_t s);
 // the map -> rho conversion, overflow and zeroing of R1 alone (tensor-core precisions)
-void launch_map_rho(const SpectralArgs &a, size_t mn, float *rho, cudaStream_t s);
+// (hi, lo: also the BF16x3 solve's parts of rho, or nullptr)
+void launch_map_rho(const SpectralArgs &a, size_t mn, float *rho, void *hi, void *lo, cudaStream_t s);
 cudaError_t spectral_prepare();
 // tensor-core form of the spectral solve (k_dctgemm.cu): kind 0 TF32, 1 BF16x3
 DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cudaStream_t stream,
                             std::string &err);
+bool dctgemm_input_parts(const DctGemmPlan &P, void **hi, void **lo);
 cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status, cudaStream_t s);
 void dctgemm_destroy(DctGemmPlan *P);
 cudaError_t place_prepare();   // opt the density scatter into its dynamic shared memory

@@ -14,21 +14,32 @@
 // K contiguous): the first GEMM of each 2-D transform stores its result
 // transposed, which is the K-major operand of the second.
 //
-// GEMM kernel: one CTA of 128 threads per 128 x BN output tile (BN = 128, or 64
-// for the launches with a single contraction, which then fill the SMs).  Thread 0
-// issues TMA tile loads (128-byte swizzle) into an S-stage shared-memory ring;
-// thread 32 issues the tcgen05.mma instructions into a 128-column FP32
-// accumulator (BN columns) in tensor memory and releases each stage with tcgen05.commit; the
-// four warps then read the accumulator (tcgen05.ld, one row per thread) and
-// store it.  Every mbarrier wait is bounded (status bit kStatusWaitTimeout).
+// A launch whose result is wanted transposed (the K-major operand of the next one)
+// exchanges its operands instead: (A B^T)^T = B A^T, so every result is stored by rows.
+//
+// GEMM kernel: persistent CTAs, one per SM, over 128 x BN output tiles (tile_width).
+// Thread 0 issues TMA tile loads (128-byte swizzle) into a ring of shared-memory
+// stages; thread 32 issues the tcgen05.mma instructions into one of two FP32
+// accumulators of BN columns in tensor memory and releases each stage with
+// tcgen05.commit; eight warps read the other accumulator (tcgen05.ld, a row per
+// thread) and store it meanwhile.  Every mbarrier wait is bounded (status bit
+// kStatusWaitTimeout).
+//
+// What bounds it: up to 1024^2 the operands' way from L2 (0.3 us per 32 columns of K
+// with 24 KB per CTA and step, 10 TB/s over 128 CTAs); at 2048^2 the tensor cores with
+// their last wave (2.5 waves of 128 x 256 tiles for three maps).  Measured against one
+// CTA of 128 threads per tile with a shared-memory transpose in its epilogue, us per
+// solve on the device: 2048^2 BF16x3 with the potential 476 -> 317, TF32 290 -> 229;
+// 1024^2 96 -> 80 and 66 -> 64; 1024 x 512 TF32 56 -> 50; 512^2 BF16x3 50 -> 39.  Same bits.
 #include <cuda.h>
 #include <cudaTypedefs.h>
-#include <cuda_bf16.h>
 #include <math.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
+#include "bf16_split.cuh"
 #include "bulk_copy.cuh"
 #include "erp_internal.cuh"
 
@@ -45,14 +56,16 @@ struct GemmMaps {            // per z: A (hi, lo) and B (hi, lo); lo only for BF
 
 struct GemmEpi {
     int mode;                // 0: plain store, 1: weighted spectra (planes)
-    int transpose;           // plain: store C^T
     int split;               // store bf16 hi/lo instead of fp32
+    int lo_first;            // BF16x3: the product lo.hi before hi.lo
+    int wide;                // every output row starts on a 32-byte boundary
     int nplanes;             // weighted mode: planes x, y (, p)
     float alpha;             // scale applied before storing
     int ldc;                 // row stride of the stored matrix (elements)
     void *out[3][2];         // per z (plain) or per plane (weighted): fp32 or bf16 hi, bf16 lo
     const float *wu, *wv;    // weighted mode: frequencies of rows (wu) and columns (wv)
     int *status;             // bounded-wait failure flag (kStatusWaitTimeout)
+    int status_on_host;      // it is page-locked host memory: only ever set, by a plain store
 };
 
 // ---- PTX wrappers (tcgen05, TMA) ----
@@ -123,196 +136,272 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 bytes to a 32-byte boundary in one instruction
+__device__ __forceinline__ void store_sector(void *p, const uint32_t (&r)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void store_words(uint32_t *p, const uint32_t (&r)[8], int wide) {
+    if (wide) {
+        store_sector(p, r);
+    } else {
+        reinterpret_cast<uint4 *>(p)[0] = make_uint4(r[0], r[1], r[2], r[3]);
+        reinterpret_cast<uint4 *>(p)[1] = make_uint4(r[4], r[5], r[6], r[7]);
+    }
+}
+// 32 consecutive elements of a matrix from element `at` on: fp32, or bf16 hi and lo
+__device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, const float (&x)[32], int split, int wide) {
+    if (!split) {
+        uint32_t *o = static_cast<uint32_t *>(out[0]) + at;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t r[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) r[k] = __float_as_uint(x[8 * q + k]);
+            store_words(o + 8 * q, r, wide);
+        }
+        return;
+    }
+    uint32_t *oh = static_cast<uint32_t *>(out[0]) + at / 2, *ol = static_cast<uint32_t *>(out[1]) + at / 2;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        uint32_t h[8], l[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float a = x[16 * q + 2 * k], b = x[16 * q + 2 * k + 1];
+            __nv_bfloat162 hi, lo;
+            split_pair(a, b, hi, lo);
+            memcpy(&h[k], &hi, 4);
+            memcpy(&l[k], &lo, 4);
+        }
+        store_words(oh + 8 * q, h, wide);
+        store_words(ol + 8 * q, l, wide);
+    }
+}
+
 // Stage ring: A tile 128 x 128 bytes, B tile BN x 128 bytes (+ the lo parts
-// for BF16x3).
+// for BF16x3), as many stages as fit in 200 KB: one CTA per SM, which may then use
+// all of the SM's tensor memory.  TF32 up to 128 columns: 100 KB, two CTAs per SM with
+// 2 BN columns of tensor memory each (more stages measured no faster, and launches of
+// short grids start later with 200 KB: 1024 x 512 solve 52.6 against 50.3 us).
 template <int KIND, int BN>
 struct GemmCfg {
     static constexpr int kABytes = kTile * 128, kBBytes = BN * 128;
     static constexpr int kStageBytes = (KIND == 0 ? 1 : 2) * (kABytes + kBBytes);
-    // TF32: 3-4 stages (96-99 KB), so two CTAs share an SM and the 128 x 128
-    // launches of a 2048^2 solve run in one wave (6 stages: 311 -> 3 stages: 247 us
-    // per solve, same bits); BF16 hi/lo stages are twice as large (one CTA per SM)
-    static constexpr int kStages = KIND == 0 ? (BN == 128 ? 3 : 4) : (BN == 128 ? 3 : 4);
+    static constexpr int kBudget = KIND == 0 && BN <= 128 ? 100 : 200;
+    static constexpr int kStages = kBudget * 1024 / kStageBytes;
     static constexpr int kBK = KIND == 0 ? 32 : 64;             // K elements per stage (128 bytes)
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
 };
+constexpr int kGemmThreads = 320;   // TMA warp, MMA warp, eight epilogue warps
 
 template <int KIND, int BN>
-__global__ void __launch_bounds__(128, 1) k_gemm_nt(const __grid_constant__ GemmMaps maps, GemmEpi epi, int K) {
+__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_nt(const __grid_constant__ GemmMaps maps, GemmEpi epi, int K,
+                                                             int tiles_m, int tiles_n, int total) {
     using Cfg = GemmCfg<KIND, BN>;
     constexpr int S = Cfg::kStages;
     extern __shared__ uint8_t dsm[];
-    __shared__ __align__(8) uint64_t full[S], empty[S], done;
+    __shared__ __align__(8) uint64_t full[S], empty[S], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int z = blockIdx.z;
-    const int tile_m = blockIdx.y * kTile, tile_n = blockIdx.x * BN;
     const int KT = K / Cfg::kBK;
 
-    if (warp == 0) {   // BN accumulator columns; at most two CTAs per SM, so at most 256 of the 512 columns
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base)),
-                     "r"(BN)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 32) {
-        for (int s = 0; s < S; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        mbar_init(&done, 1);
-        failed = 0;
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = tmem_base;
     // stage layout: A hi | B hi | A lo | B lo
     auto tile = [&](int s, int op) {
         const size_t off = (op & 1) ? Cfg::kABytes : 0;
         return base + (size_t)s * Cfg::kStageBytes + (size_t)(op >> 1) * (Cfg::kABytes + Cfg::kBBytes) + off;
     };
+    // this CTA's output tiles: blockIdx.x, blockIdx.x + gridDim.x, ... of z-major rows of tiles
+    struct Tile {
+        int z, m, n;
+    };
+    auto tile_at = [&](int t) {
+        const int z = t / (tiles_m * tiles_n), r = t - z * tiles_m * tiles_n;
+        const int tm = r / tiles_n;
+        return Tile{z, tm * kTile, (r - tm * tiles_n) * BN};
+    };
 
-    if (tid == 0) {   // TMA producer
-        for (int kt = 0; kt < KT; ++kt) {
-            const int s = kt % S;
-            const uint32_t ph = (uint32_t)(kt / S) & 1u;
-            if (!mbar_wait(&empty[s], ph ^ 1u)) { failed = 1; break; }
-            mbar_expect_tx(&full[s], (uint32_t)Cfg::kStageBytes);
-            const int k0 = kt * Cfg::kBK;
-            tma_load_2d(tile(s, 0), &maps.a[z][0], k0, tile_m, &full[s]);
-            tma_load_2d(tile(s, 1), &maps.b[z][0], k0, tile_n, &full[s]);
-            if (KIND == 1) {
-                tma_load_2d(tile(s, 2), &maps.a[z][1], k0, tile_m, &full[s]);
-                tma_load_2d(tile(s, 3), &maps.b[z][1], k0, tile_n, &full[s]);
-            }
+    auto load_stage = [&](const Tile &tl, int kt, int s) {
+        mbar_expect_tx(&full[s], (uint32_t)Cfg::kStageBytes);
+        const int k0 = kt * Cfg::kBK;
+        tma_load_2d(tile(s, 0), &maps.a[tl.z][0], k0, tl.m, &full[s]);
+        tma_load_2d(tile(s, 1), &maps.b[tl.z][0], k0, tl.n, &full[s]);
+        if (KIND == 1) {
+            tma_load_2d(tile(s, 2), &maps.a[tl.z][1], k0, tl.m, &full[s]);
+            tma_load_2d(tile(s, 3), &maps.b[tl.z][1], k0, tl.n, &full[s]);
         }
-    } else if (tid == 32) {   // MMA issuer
-        for (int kt = 0; kt < KT; ++kt) {
-            const int s = kt % S;
-            const uint32_t ph = (uint32_t)(kt / S) & 1u;
-            if (!mbar_wait(&full[s], ph)) { failed = 1; break; }
-            tc_fence_after();
-            const uint32_t a0 = smem_addr(tile(s, 0)), b0 = smem_addr(tile(s, 1));
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {   // 4 x 32 bytes of K per 128-byte row
-                const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-                if (KIND == 0) {
-                    mma_issue<0, BN>(tmem, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), acc);
-                } else {
-                    const uint32_t a1 = smem_addr(tile(s, 2)), b1 = smem_addr(tile(s, 3));
-                    mma_issue<1, BN>(tmem, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), acc);   // hi.hi
-                    mma_issue<1, BN>(tmem, sw128_desc(a0 + 32 * kk), sw128_desc(b1 + 32 * kk), 1u);    // hi.lo
-                    mma_issue<1, BN>(tmem, sw128_desc(a1 + 32 * kk), sw128_desc(b0 + 32 * kk), 1u);    // lo.hi
-                }
-            }
-            mma_commit(&empty[s]);   // the stage is free once these MMAs have read it
+    };
+
+    // The first tile's first stages are on their way while the tensor memory is being
+    // allocated (more of them would hold up the barrier below).
+    const int ahead = min(2, KT);
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
         }
-        mma_commit(&done);
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&acc_full[k], 1);
+            mbar_init(&acc_empty[k], 8);   // one arrival per epilogue warp
+        }
+        failed = 0;
+        const Tile first = tile_at(blockIdx.x);
+        for (int kt = 0; kt < ahead; ++kt) load_stage(first, kt, kt);
     }
-    __syncwarp();
-    const bool ok = mbar_wait(&done, 0u);
-    if (!ok && lane == 0) failed = 1;
-    tc_fence_after();
-    if (ok) {
-        // The stage ring is idle now (every MMA has completed): for the weighted
-        // spectra and split outputs each warp transposes its 32 x 32 chunks
-        // through a 32 x 33 buffer there, so that the many narrow row-major
-        // stores go out with consecutive columns across the lanes; plain fp32
-        // rows use 128-bit stores of the thread's own row.
-        float *buf = reinterpret_cast<float *>(base) + warp * (32 * 33);
-        const int r = warp * 32 + lane;   // this thread's accumulator row (TMEM lane)
-        const int gr = tile_m + r;
-        const float al = epi.alpha;
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-            float v[32];
-            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (epi.mode == 0 && epi.transpose) {   // C^T: lanes hold consecutive rows already
-                if (!epi.split) {
-                    float *o = static_cast<float *>(epi.out[z][0]);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) o[(size_t)(tile_n + c0 + j) * epi.ldc + gr] = al * v[j];
-                } else {
-                    __nv_bfloat16 *oh = static_cast<__nv_bfloat16 *>(epi.out[z][0]);
-                    __nv_bfloat16 *ol = static_cast<__nv_bfloat16 *>(epi.out[z][1]);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const size_t idx = (size_t)(tile_n + c0 + j) * epi.ldc + gr;
-                        const float x = al * v[j];
-                        const __nv_bfloat16 h = __float2bfloat16_rn(x);
-                        oh[idx] = h;
-                        ol[idx] = __float2bfloat16_rn(x - __bfloat162float(h));
-                    }
-                }
-                continue;
-            }
-            if (epi.mode == 0 && !epi.split) {   // plain fp32 rows: the thread's 32 columns, 128-bit stores
-                float4 *d = reinterpret_cast<float4 *>(static_cast<float *>(epi.out[z][0]) + (size_t)gr * epi.ldc +
-                                                       tile_n + c0);
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    d[q] = make_float4(al * v[4 * q], al * v[4 * q + 1], al * v[4 * q + 2], al * v[4 * q + 3]);
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) buf[lane * 33 + j] = v[j];
-            __syncwarp();
-            const int gc = tile_n + c0 + lane;
-            const float wv = epi.mode == 1 ? epi.wv[gc] : 0.0f;
-            const bool three = epi.nplanes > 2;
-            for (int rr = 0; rr < 32; ++rr) {
-                const int gr2 = tile_m + warp * 32 + rr;
-                const size_t idx = (size_t)gr2 * epi.ldc + gc;
-                const float x = al * buf[rr * 33 + lane];
-                if (epi.mode == 0) {
-                    if (!epi.split) {
-                        static_cast<float *>(epi.out[z][0])[idx] = x;
-                    } else {
-                        const __nv_bfloat16 h = __float2bfloat16_rn(x);
-                        static_cast<__nv_bfloat16 *>(epi.out[z][0])[idx] = h;
-                        static_cast<__nv_bfloat16 *>(epi.out[z][1])[idx] = __float2bfloat16_rn(x - __bfloat162float(h));
-                    }
-                } else {   // weighted spectra: row u = gr2, column v = gc (planes x, y, p)
-                    const float wu = epi.wu[gr2];
-                    const float k2 = __fadd_rn(__fmul_rn(wu, wu), __fmul_rn(wv, wv));
-                    const float ik = (gr2 == 0 && gc == 0) ? 0.0f : __frcp_rn(k2);
-                    const float px = x * (0.5f * wu * ik), py = x * (0.5f * wv * ik), pp = x * ik;
-                    if (!epi.split) {
-                        static_cast<float *>(epi.out[0][0])[idx] = px;
-                        static_cast<float *>(epi.out[1][0])[idx] = py;
-                        if (three) static_cast<float *>(epi.out[2][0])[idx] = pp;
-                    } else {
-                        __nv_bfloat16 h = __float2bfloat16_rn(px);
-                        static_cast<__nv_bfloat16 *>(epi.out[0][0])[idx] = h;
-                        static_cast<__nv_bfloat16 *>(epi.out[0][1])[idx] = __float2bfloat16_rn(px - __bfloat162float(h));
-                        h = __float2bfloat16_rn(py);
-                        static_cast<__nv_bfloat16 *>(epi.out[1][0])[idx] = h;
-                        static_cast<__nv_bfloat16 *>(epi.out[1][1])[idx] = __float2bfloat16_rn(py - __bfloat162float(h));
-                        if (three) {
-                            h = __float2bfloat16_rn(pp);
-                            static_cast<__nv_bfloat16 *>(epi.out[2][0])[idx] = h;
-                            static_cast<__nv_bfloat16 *>(epi.out[2][1])[idx] = __float2bfloat16_rn(pp - __bfloat162float(h));
-                        }
-                    }
-                }
-            }
-            __syncwarp();
-        }
+    if (warp == 1) {   // two accumulators of BN columns; one CTA per SM, so all 512 columns may be taken
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base)),
+                     "r"(2 * BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
-    if (failed && tid == 0 && epi.status) atomicOr(epi.status, kStatusWaitTimeout);
-    if (warp == 0) {
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+
+    if (tid == 0) {   // TMA producer
+        int it = ahead, kt = ahead;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x, kt = 0) {
+            const Tile tl = tile_at(t);
+            for (; kt < KT; ++kt, ++it) {
+                const int s = it % S;
+                ok = mbar_wait(&empty[s], ((uint32_t)(it / S) & 1u) ^ 1u);
+                if (!ok) break;
+                load_stage(tl, kt, s);
+            }
+        }
+        if (!ok) {   // a wait ran out: the copies in flight land before the block leaves
+            failed = 1;
+            for (int k = it > S ? it - S : 0; k < it; ++k) mbar_wait(&full[k % S], (uint32_t)(k / S) & 1u);
+        }
+    } else if (tid == 32) {   // MMA issuer
+        int it = 0, lt = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
+            const int buf = lt & 1;
+            if (!mbar_wait(&acc_empty[buf], (((uint32_t)lt >> 1) & 1u) ^ 1u)) { failed = 1; break; }
+            tc_fence_after();
+            const uint32_t acc_at = tmem + (uint32_t)(buf * BN);
+            bool ok = true;
+            for (int kt = 0; kt < KT; ++kt, ++it) {
+                const int s = it % S;
+                const uint32_t ph = (uint32_t)(it / S) & 1u;
+                if (!mbar_wait(&full[s], ph)) { failed = 1; ok = false; break; }
+                tc_fence_after();
+                const uint32_t a0 = smem_addr(tile(s, 0)), b0 = smem_addr(tile(s, 1));
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {   // 4 x 32 bytes of K per 128-byte row
+                    const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
+                    if (KIND == 0) {
+                        mma_issue<0, BN>(acc_at, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), acc);
+                    } else {
+                        const uint32_t a1 = smem_addr(tile(s, 2)), b1 = smem_addr(tile(s, 3));
+                        const uint32_t ax = epi.lo_first ? a1 : a0, bx = epi.lo_first ? b0 : b1;
+                        const uint32_t ay = epi.lo_first ? a0 : a1, by = epi.lo_first ? b1 : b0;
+                        mma_issue<1, BN>(acc_at, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), acc);   // hi.hi
+                        mma_issue<1, BN>(acc_at, sw128_desc(ax + 32 * kk), sw128_desc(bx + 32 * kk), 1u);    // hi.lo
+                        mma_issue<1, BN>(acc_at, sw128_desc(ay + 32 * kk), sw128_desc(by + 32 * kk), 1u);    // lo.hi
+                    }
+                }
+                mma_commit(&empty[s]);   // the stage is free once these MMAs have read it
+            }
+            mma_commit(&acc_full[buf]);
+            if (!ok) break;
+        }
+    } else if (warp >= 2) {
+        // Epilogue: warps w and w + 4 share the TMEM lanes of quarter w mod 4 and take
+        // alternate blocks of 32 columns.  Each thread holds 32 columns of its row at a
+        // time and stores them itself, a 32-byte sector per instruction (16 bytes where
+        // a caller's buffer allows no more): no staging, and the weights of a row share
+        // its wu.  The next tile's products run meanwhile in the other accumulator.
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const float al = epi.alpha;
+        int lt = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
+            const Tile tl = tile_at(t);
+            const int buf = lt & 1;
+            const int gr = tl.m + quarter * 32 + lane;   // this thread's row
+            const float wu = epi.mode == 1 ? epi.wu[gr] : 0.0f;
+            const bool ready = mbar_wait(&acc_full[buf], ((uint32_t)lt >> 1) & 1u);
+            if (!__all_sync(0xffffffffu, ready)) {   // one decision per warp
+                failed = 1;
+                break;
+            }
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = 32 * half; c0 < BN; c0 += 64) {
+                float v[32];
+                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), v);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] *= al;
+                const size_t at = (size_t)gr * epi.ldc + tl.n + c0;
+                if (epi.mode == 0) {
+                    store_row(epi.out[tl.z], at, v, epi.split, epi.wide);
+                    continue;
+                }
+                // weighted spectra: row u = gr, column gc (planes x, y, p)
+                float px[32], py[32];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float4 w4 = __ldg(reinterpret_cast<const float4 *>(epi.wv + tl.n + c0) + q);
+                    const float wv4[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int j = 4 * q + e;
+                        const float wv = wv4[e];
+                        const float k2 = __fadd_rn(__fmul_rn(wu, wu), __fmul_rn(wv, wv));
+                        const float ik = (gr | (tl.n + c0 + j)) == 0 ? 0.0f : __frcp_rn(k2);
+                        const float x = v[j];
+                        px[j] = x * (0.5f * wu * ik);
+                        py[j] = x * (0.5f * wv * ik);
+                        v[j] = x * ik;
+                    }
+                }
+                store_row(epi.out[0], at, px, epi.split, epi.wide);
+                store_row(epi.out[1], at, py, epi.split, epi.wide);
+                if (epi.nplanes > 2) store_row(epi.out[2], at, v, epi.split, epi.wide);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (failed && tid == 0 && epi.status) {
+        if (epi.status_on_host) *(volatile int *)epi.status = kStatusWaitTimeout;
+        else atomicOr(epi.status, kStatusWaitTimeout);
+    }
+    if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
     }
 }
 
+// hi and lo of the caller's input; VEC: four elements per thread from a 16-byte boundary
+template <bool VEC>
 __global__ void k_split_bf16(size_t count, const float *__restrict__ src, __nv_bfloat16 *__restrict__ hi,
                              __nv_bfloat16 *__restrict__ lo) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    if (VEC) {
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count / 4; i += step) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(src) + i);
+            __nv_bfloat162 h[2], l[2];
+            split_pair(v.x, v.y, h[0], l[0]);
+            split_pair(v.z, v.w, h[1], l[1]);
+            uint2 ph, pl;
+            memcpy(&ph, h, 8);
+            memcpy(&pl, l, 8);
+            reinterpret_cast<uint2 *>(hi)[i] = ph;
+            reinterpret_cast<uint2 *>(lo)[i] = pl;
+        }
+        return;
+    }
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += step) {
         const float v = src[i];
         const __nv_bfloat16 h = __float2bfloat16_rn(v);
         hi[i] = h;
@@ -365,11 +454,11 @@ struct DctGemmPlan {
     GemmOperand Aw[3];                    // [m][n] weighted spectra x, y, p
     GemmOperand Zkt[3];                   // [n][m] after the first inverse contraction
     float *wu = nullptr, *wv = nullptr;
-    int *status = nullptr;
-    int *h_status = nullptr;              // pinned mirror, refreshed after every solve
+    int *h_status = nullptr;              // page-locked: set by a launch whose bounded wait ran out
     std::vector<void *> owned;
     const void *rho_cached = nullptr;     // TF32: the rho the first map was built for
-    GemmMaps g1, g2, g3, g4;
+    GemmMaps g1, g2, g3[2], g4[2];        // G3, G4: without and with the potential
+    int bn[2], bn3[2], bn4[2];            // their output tiles' widths
 };
 
 static bool alloc_operand(DctGemmPlan &P, GemmOperand &o, size_t count) {
@@ -413,6 +502,30 @@ void dctgemm_destroy(DctGemmPlan *P) {
     delete P;
 }
 
+// Width of the output tiles of a launch: the narrowest for which every tile has an SM
+// of its own; else 256, whose operand reads from shared memory keep up with the tensor
+// cores (per 16 columns of K, 128 bytes a cycle at 128 columns, 96 at 256).
+// Measured, us per launch at widths 32 / 64 / 128 / 256:
+//   BF16x3 512^2, K 512 (32 has 64 tiles)       8.8 / 9.3 / 10.4 / 14.7
+//   TF32 1024^2 (64 has 128 tiles)               23.8 / 14.7 / 15.4 / 17.3
+//   BF16x3 2048 x 1024 (128 has 128 tiles)       40.2 / 23.1 / 15.4 / 23.7
+//   BF16x3 2048^2 (256 has 128 tiles)            128 / 76 / 42.5 / 40.4, three maps 376 / 201 / 117 / 108
+static int tile_width(int M, int N, int Z) {
+    for (int bn : {32, 64, 128})
+        if ((long long)(M / kTile) * (N / bn) * Z <= 152) return bn;
+    return N % 256 ? 128 : 256;
+}
+
+template <int KIND, int BN>
+static bool prepare_gemm() {
+    return cudaFuncSetAttribute(k_gemm_nt<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)GemmCfg<KIND, BN>::kSmem) == cudaSuccess;
+}
+static bool prepare_gemms() {
+    return prepare_gemm<0, 32>() && prepare_gemm<0, 64>() && prepare_gemm<0, 128>() && prepare_gemm<0, 256>() &&
+           prepare_gemm<1, 32>() && prepare_gemm<1, 64>() && prepare_gemm<1, 128>() && prepare_gemm<1, 256>();
+}
+
 // transform matrices (FP64 closed forms), buffers and the tensor maps that do
 // not depend on the caller's input
 DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cudaStream_t stream,
@@ -425,14 +538,7 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
         err = "cuTensorMapEncodeTiled is not available from the driver";
         return nullptr;
     }
-    if (cudaFuncSetAttribute(k_gemm_nt<0, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)GemmCfg<0, 64>::kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_gemm_nt<0, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)GemmCfg<0, 128>::kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_gemm_nt<1, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)GemmCfg<1, 64>::kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_gemm_nt<1, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)GemmCfg<1, 128>::kSmem) != cudaSuccess) {
+    if (!prepare_gemms()) {
         err = "cudaFuncSetAttribute failed";
         return nullptr;
     }
@@ -469,23 +575,26 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
     if (ok) P->owned.push_back(P->wu);
     ok = ok && cudaMalloc(&P->wv, sizeof(float) * n) == cudaSuccess;
     if (ok) P->owned.push_back(P->wv);
-    ok = ok && cudaMalloc(&P->status, sizeof(int)) == cudaSuccess;
-    if (ok) P->owned.push_back(P->status);
     ok = ok && cudaMallocHost((void **)&P->h_status, sizeof(int)) == cudaSuccess;
     if (ok) *P->h_status = 0;
     ok = ok && cudaMemcpy(P->wu, hu.data(), sizeof(float) * m, cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(P->wv, hv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemset(P->status, 0, sizeof(int)) == cudaSuccess;
+         cudaMemcpy(P->wv, hv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) == cudaSuccess;
     // maps: G1 A = rho (per call for TF32, rho2 for BF16x3), B = C_n;  G2 A = C_m, B = Zt;
     // G3 A = Aw[k], B = D_n / S_n / D_n;  G4 A = S_m / D_m / D_m, B = Zkt[k]
     // G1 and G2 (one contraction per launch) use 128 x 64 tiles: twice the CTAs
-    ok = ok && set_maps(*P, P->g1.b[0], P->Cn, n, n, 64) && set_maps(*P, P->g2.a[0], P->Cm, m, m) &&
-         set_maps(*P, P->g2.b[0], P->Zt, n, m, 64);
-    if (ok && kind == 1) ok = set_maps(*P, P->g1.a[0], P->rho2, m, n);
+    P->bn[0] = tile_width(n, m, 1);
+    P->bn[1] = tile_width(m, n, 1);
+    ok = ok && set_maps(*P, P->g1.a[0], P->Cn, n, n) && set_maps(*P, P->g2.a[0], P->Cm, m, m) &&
+         set_maps(*P, P->g2.b[0], P->Zt, n, m, P->bn[1]);
+    if (ok && kind == 1) ok = set_maps(*P, P->g1.b[0], P->rho2, m, n, P->bn[0]);
     const GemmOperand *b3[3] = {&P->Dn, &P->Sn, &P->Dn}, *a4[3] = {&P->Sm, &P->Dm, &P->Dm};
-    for (int k = 0; ok && k < 3; ++k)
-        ok = set_maps(*P, P->g3.a[k], P->Aw[k], m, n) && set_maps(*P, P->g3.b[k], *b3[k], n, n) &&
-             set_maps(*P, P->g4.a[k], *a4[k], m, m) && set_maps(*P, P->g4.b[k], P->Zkt[k], n, m);
+    for (int v = 0; v < 2; ++v) {   // without and with the potential
+        P->bn3[v] = tile_width(n, m, 2 + v);
+        P->bn4[v] = tile_width(m, n, 2 + v);
+        for (int k = 0; ok && k < 2 + v; ++k)
+            ok = set_maps(*P, P->g3[v].a[k], *b3[k], n, n) && set_maps(*P, P->g3[v].b[k], P->Aw[k], m, n, P->bn3[v]) &&
+                 set_maps(*P, P->g4[v].a[k], *a4[k], m, m) && set_maps(*P, P->g4[v].b[k], P->Zkt[k], n, m, P->bn4[v]);
+    }
     if (!ok) {
         err = "tensor-core solve set-up failed";
         dctgemm_destroy(P);
@@ -496,26 +605,36 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
 
 template <int KIND, int BN>
 static cudaError_t launch_gemm(const GemmMaps &maps, const GemmEpi &epi, int M, int N, int K, int Z, cudaStream_t s) {
-    dim3 grid(N / BN, M / kTile, Z);
-    k_gemm_nt<KIND, BN><<<grid, 128, GemmCfg<KIND, BN>::kSmem, s>>>(maps, epi, K);
+    const int tm = M / kTile, tn = N / BN, total = tm * tn * Z;
+    k_gemm_nt<KIND, BN><<<std::min(total, 152), kGemmThreads, GemmCfg<KIND, BN>::kSmem, s>>>(maps, epi, K, tm, tn, total);
     return cudaGetLastError();
 }
 
 static cudaError_t run_gemm(const DctGemmPlan &P, const GemmMaps &maps, const GemmEpi &epi, int M, int N, int K,
                             int Z, int bn, cudaStream_t s) {
-    if (bn == 64)
-        return P.kind == 0 ? launch_gemm<0, 64>(maps, epi, M, N, K, Z, s) : launch_gemm<1, 64>(maps, epi, M, N, K, Z, s);
-    return P.kind == 0 ? launch_gemm<0, 128>(maps, epi, M, N, K, Z, s)
-                       : launch_gemm<1, 128>(maps, epi, M, N, K, Z, s);
+#define G(B) P.kind == 0 ? launch_gemm<0, B>(maps, epi, M, N, K, Z, s) : launch_gemm<1, B>(maps, epi, M, N, K, Z, s)
+    if (bn == 32) return G(32);
+    if (bn == 64) return G(64);
+    if (bn == 128) return G(128);
+    return G(256);
+}
+
+// Where a BF16x3 solve reads its input's hi and lo parts from; a caller that writes them
+// itself passes rho = nullptr to dctgemm_solve.  False: the plan is TF32.
+bool dctgemm_input_parts(const DctGemmPlan &P, void **hi, void **lo) {
+    *hi = P.rho2.p[0];
+    *lo = P.rho2.p[1];
+    return P.kind == 1;
 }
 
 // fx, fy (, psi) = Poisson solve of rho: four contraction launches (+ the split
 // of rho).  Returns cudaErrorTimeout when a bounded wait of an earlier solve
-// on this plan ran out (seen through the pinned mirror of the status word).
+// on this plan ran out.
 //
 // status: where the contractions report a bounded wait that ran out; nullptr
-// uses the plan's own word and its pinned mirror (a placement context passes
-// its DevState status, read by the host with the rest of the state).
+// uses the plan's own word, in page-locked host memory that the device writes (a
+// placement context passes its DevState status, read by the host with the rest of
+// the state).
 cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy, float *psi, int *status, cudaStream_t s) {
     if (!status && *(volatile int *)P.h_status) return cudaErrorTimeout;
     const int m = P.m, n = P.n, nk = psi ? 3 : 2;
@@ -523,38 +642,47 @@ cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy
     const bool split = P.kind == 1;
     cudaError_t e = cudaSuccess;
     if (split) {
-        k_split_bf16<<<152 * 8, 256, 0, s>>>(mn, rho, (__nv_bfloat16 *)P.rho2.p[0],
-                                                   (__nv_bfloat16 *)P.rho2.p[1]);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (rho) {   // else the caller has filled the parts (dctgemm_input_parts)
+            const bool vec = (reinterpret_cast<uintptr_t>(rho) & 15) == 0;   // mn is a multiple of 4
+            (vec ? k_split_bf16<true> : k_split_bf16<false>)<<<152 * 8, 256, 0, s>>>(
+                mn, rho, (__nv_bfloat16 *)P.rho2.p[0], (__nv_bfloat16 *)P.rho2.p[1]);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
     } else if (rho != P.rho_cached) {
-        if (!make_map(&P.g1.a[0][0], rho, m, n, false)) return cudaErrorInvalidValue;
-        P.g1.a[0][1] = P.g1.a[0][0];
+        if (!make_map(&P.g1.b[0][0], rho, m, n, false, P.bn[0])) return cudaErrorInvalidValue;
+        P.g1.b[0][1] = P.g1.b[0][0];
         P.rho_cached = rho;
     }
     GemmEpi ep;
     memset(&ep, 0, sizeof ep);
-    ep.status = status ? status : P.status;
+    ep.status = status ? status : P.h_status;
+    ep.status_on_host = status ? 0 : 1;
     ep.split = split ? 1 : 0;
-    // G1: Z = rho C_n^T, stored transposed [n][m]
-    ep.mode = 0; ep.transpose = 1; ep.alpha = 1.0f; ep.ldc = m;
+    ep.wide = 1;   // the plan's own buffers
+    // G1: Z^T = C_n rho^T [n][m] (the operands' order gives the transpose; lo_first keeps
+    // the order of the products rho hi . C_n lo, rho lo . C_n hi)
+    ep.mode = 0; ep.lo_first = 1; ep.alpha = 1.0f; ep.ldc = m;
     ep.out[0][0] = P.Zt.p[0]; ep.out[0][1] = P.Zt.p[1];
-    if ((e = run_gemm(P, P.g1, ep, m, n, n, 1, 64, s)) != cudaSuccess) return e;
+    if ((e = run_gemm(P, P.g1, ep, n, m, n, 1, P.bn[0], s)) != cudaSuccess) return e;
     // G2: A = (4/mn) C_m Z, written as the weighted spectra [m][n]
-    ep.mode = 1; ep.transpose = 0; ep.alpha = (float)(4.0 / ((double)m * (double)n)); ep.ldc = n;
+    ep.mode = 1; ep.lo_first = 0; ep.alpha = (float)(4.0 / ((double)m * (double)n)); ep.ldc = n;
     ep.nplanes = nk; ep.wu = P.wu; ep.wv = P.wv;
     for (int k = 0; k < 3; ++k) { ep.out[k][0] = P.Aw[k].p[0]; ep.out[k][1] = P.Aw[k].p[1]; }
-    if ((e = run_gemm(P, P.g2, ep, m, n, m, 1, 64, s)) != cudaSuccess) return e;
-    // G3: Z_k = Aw_k (D_n | S_n | D_n)^T, stored transposed [n][m]
-    ep.mode = 0; ep.transpose = 1; ep.alpha = 1.0f; ep.ldc = m; ep.nplanes = 0;
+    if ((e = run_gemm(P, P.g2, ep, m, n, m, 1, P.bn[1], s)) != cudaSuccess) return e;
+    // G3: Z_k^T = (D_n | S_n | D_n) Aw_k^T [n][m]
+    ep.mode = 0; ep.lo_first = 1; ep.alpha = 1.0f; ep.ldc = m; ep.nplanes = 0;
     for (int k = 0; k < 3; ++k) { ep.out[k][0] = P.Zkt[k].p[0]; ep.out[k][1] = P.Zkt[k].p[1]; }
-    if ((e = run_gemm(P, P.g3, ep, m, n, n, nk, 128, s)) != cudaSuccess) return e;
-    // G4: field_x = S_m Z_x, field_y = D_m Z_y, psi = D_m Z_p, fp32 [m][n]
-    ep.split = 0; ep.transpose = 0; ep.ldc = n;
+    if ((e = run_gemm(P, P.g3[nk - 2], ep, n, m, n, nk, P.bn3[nk - 2], s)) != cudaSuccess) return e;
+    // G4: field_x = S_m Z_x, field_y = D_m Z_y, psi = D_m Z_p, fp32 [m][n], the caller's buffers
+    ep.split = 0; ep.lo_first = 0; ep.ldc = n;
     float *outs[3] = {fx, fy, psi};
-    for (int k = 0; k < 3; ++k) { ep.out[k][0] = outs[k]; ep.out[k][1] = nullptr; }
-    if ((e = run_gemm(P, P.g4, ep, m, n, m, nk, 128, s)) != cudaSuccess) return e;
-    if (status) return cudaSuccess;
-    return cudaMemcpyAsync(P.h_status, P.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+    for (int k = 0; k < nk; ++k) {
+        ep.out[k][0] = outs[k];
+        ep.out[k][1] = nullptr;
+        if (reinterpret_cast<uintptr_t>(outs[k]) & 31) ep.wide = 0;
+    }
+    if ((e = run_gemm(P, P.g4[nk - 2], ep, m, n, m, nk, P.bn4[nk - 2], s)) != cudaSuccess) return e;
+    return cudaSuccess;
 }
 
 }  // namespace erp

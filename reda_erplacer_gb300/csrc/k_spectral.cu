@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "erp_internal.cuh"
+#include "bf16_split.cuh"
 #include "bulk_copy.cuh"
 #include "fft_pair.cuh"
 #include "fixedpoint.h"
@@ -676,23 +677,38 @@ __global__ void __launch_bounds__(PairFft<N, P>::THREADS) k_rows_inv(const __gri
 
 // The density map as rho for the tensor-core solve: the conversion of R1 (same
 // float rules, so rho is bit-identical to what the FFT path transforms), the
-// double-float overflow sum with the last-block finalize, and the map zeroing.
-__global__ void __launch_bounds__(kThreads) k_map_rho(size_t mn, unsigned long long *__restrict__ dmap,
-                                                      const float *__restrict__ initial, float fixed_inv, float coef,
-                                                      float inv_area, int zero_map, float *__restrict__ rho,
+// double-float overflow sum, and the map zeroing, two bins per thread; with hi and lo
+// also the BF16x3 solve's split of rho, which was a launch of its own.  512^2 bins: this
+// kernel (with its own reduction tail) and the split 8.2 + 1.8 us, now 4.8 us.
+__global__ void __launch_bounds__(kThreads) k_map_rho(size_t pairs, ulonglong2 *__restrict__ dmap,
+                                                      const float2 *__restrict__ initial, float fixed_inv, float coef,
+                                                      float inv_area, int zero_map, float2 *__restrict__ rho,
+                                                      __nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo,
                                                       double *__restrict__ partials, DevState *__restrict__ st,
                                                       double movable_area, int step) {
     __shared__ double shr[kThreads / 32];
     if (st->done) return;
     Df ovf = df_zero();
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < mn; idx += (size_t)gridDim.x * blockDim.x) {
-        const unsigned long long q = dmap[idx];
-        if (zero_map) dmap[idx] = 0ull;
-        // d = (float)sum * 2^-S + initial  (src/density.rs:231-236, fixed point)
-        const float d = __fadd_rn(__fmul_rn(fxp_u64_to_float(q), fixed_inv), initial[idx]);
-        const float o = __fsub_rn(d, coef);
-        ovf = df_add(ovf, o > 0.0f ? o : 0.0f);  // src/epotential.rs:274-276
-        rho[idx] = __fmul_rn(d, inv_area);         // src/epotential.rs:284-285
+    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < pairs; idx += (size_t)gridDim.x * blockDim.x) {
+        const ulonglong2 q = dmap[idx];
+        const float2 ini = initial[idx];
+        if (zero_map) dmap[idx] = make_ulonglong2(0ull, 0ull);
+        float r[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            // d = (float)sum * 2^-S + initial  (src/density.rs:231-236, fixed point)
+            const float d = __fadd_rn(__fmul_rn(fxp_u64_to_float(h ? q.y : q.x), fixed_inv), h ? ini.y : ini.x);
+            const float o = __fsub_rn(d, coef);
+            ovf = df_add(ovf, o > 0.0f ? o : 0.0f);  // src/epotential.rs:274-276
+            r[h] = __fmul_rn(d, inv_area);             // src/epotential.rs:284-285
+        }
+        rho[idx] = make_float2(r[0], r[1]);
+        if (hi) {
+            __nv_bfloat162 a, b;
+            split_pair(r[0], r[1], a, b);
+            hi[idx] = a;
+            lo[idx] = b;
+        }
     }
     const Df vals[1] = {block_sum(ovf, shr)};
     if (step) {
@@ -709,11 +725,14 @@ __global__ void __launch_bounds__(kThreads) k_map_rho(size_t mn, unsigned long l
     }
 }
 
-int map_rho_blocks(size_t mn) { return (int)std::min<size_t>((mn + kThreads - 1) / kThreads, 152 * 8); }
+// mn is even: both sides are multiples of 128
+int map_rho_blocks(size_t mn) { return (int)std::min<size_t>((mn / 2 + kThreads - 1) / kThreads, 152 * 8); }
 
-void launch_map_rho(const SpectralArgs &a, size_t mn, float *rho, cudaStream_t s) {
-    k_map_rho<<<map_rho_blocks(mn), kThreads, 0, s>>>(mn, a.dmap, a.initial, a.fixed_inv, a.coef, a.inv_bin_area,
-                                          a.zero_map ? 1 : 0, rho, a.partials, a.st, a.movable_area, a.step ? 1 : 0);
+void launch_map_rho(const SpectralArgs &a, size_t mn, float *rho, void *hi, void *lo, cudaStream_t s) {
+    k_map_rho<<<map_rho_blocks(mn), kThreads, 0, s>>>(
+        mn / 2, reinterpret_cast<ulonglong2 *>(a.dmap), reinterpret_cast<const float2 *>(a.initial), a.fixed_inv, a.coef,
+        a.inv_bin_area, a.zero_map ? 1 : 0, reinterpret_cast<float2 *>(rho), static_cast<__nv_bfloat162 *>(hi),
+        static_cast<__nv_bfloat162 *>(lo), a.partials, a.st, a.movable_area, a.step ? 1 : 0);
 }
 
 int ilog2(int v) {

@@ -33,3 +33,33 @@ def test_solve_buffers(m, n):
     for r in results[1:]:
         for a, b in zip(results[0], r):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("m,n", [(128, 128), (128, 2048), (2048, 128), (256, 512), (1024, 1024), (2048, 2048)])
+def test_contraction_tiles(m, n, precision):
+    """The tensor-core solve at sizes that take every tile width, one tile per SM
+    and several: the two fields are the same bits with and without the potential
+    (other widths and other tiles per SM), on 32-byte and on 16-byte boundaries
+    (other stores), and twice in a row (the ring and both accumulators in use
+    again).  (Accuracy is tested in test_gpu_parity.py.)"""
+    import torch
+    import reda_erplacer_gb300 as R
+    rng = np.random.default_rng(m + n)
+    rho = torch.from_numpy((0.7 + 0.3 * rng.random(m * n)).astype(np.float32)).cuda()
+    stream = torch.cuda.current_stream().cuda_stream
+    s = R.SpectralSolver(m, n, 1.3, 1.0, stream=stream, precision=precision)
+    results = []
+    for offset in (0, 4, 0):
+        buf = [torch.zeros(m * n + 8, dtype=torch.float32, device="cuda") for _ in range(3)]
+        at = [b[offset:offset + m * n] for b in buf]
+        for psi in (at[2].data_ptr(), None):
+            s.solve(rho.data_ptr(), at[0].data_ptr(), at[1].data_ptr(), psi)
+            torch.cuda.synchronize()
+            results.append([t.clone() for t in at])
+        for b in buf:
+            assert float(b[:offset].abs().sum()) == 0 and float(b[offset + m * n:].abs().sum()) == 0
+    s.close()
+    for r in results[1:]:
+        for a, b in zip(results[0], r):
+            assert torch.equal(a, b)
