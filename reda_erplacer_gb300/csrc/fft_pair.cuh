@@ -172,6 +172,17 @@ struct PairFft {
         if constexpr (kEarly) return ld_now(p);
         else return __ldg(p);
     }
+    // A pair of the pass before: WRITTEN in the same kernel, or by an earlier one.
+    template <bool WRITTEN>
+    static __device__ __forceinline__ float2 load_pair(const float2 *p) {
+        if constexpr (WRITTEN) {
+            float2 v;
+            asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+            return v;
+        } else {
+            return load(p);
+        }
+    }
     // v[j] = z[t + M j] in, v[e] = Z[out_index(t, e)] out.  A: N P slots, free on
     // entry (every thread of the block past its last use) and still being read by
     // other threads on return.  tw: this length's stage twiddles; w1: load_tw1's.

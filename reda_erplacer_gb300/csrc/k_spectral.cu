@@ -507,7 +507,9 @@ struct ColsP {
     float scale4;
     const DevState * st;
 };
-template <int N, int P>
+// INNER (both passes below): their input was written earlier in the same kernel, which
+// rules the read-only path out.
+template <int N, int P, bool INNER = false>
 __device__ __forceinline__ void cols_body(const ColsP &a, int bid, int nblk) {
     using F = PairFft<N, P>;
     if (a.st && a.st->done) return;
@@ -527,7 +529,7 @@ __device__ __forceinline__ void cols_body(const ColsP &a, int bid, int nblk) {
     float2 v[F::R1], w1[F::R1];
 #pragma unroll
     for (int j = 0; j < F::R1; ++j)
-        v[j] = F::load(reinterpret_cast<const float2 *>(a.t1) + ((t + j * F::M) >> 1) * n + at0);
+        v[j] = F::template load_pair<INNER>(reinterpret_cast<const float2 *>(a.t1) + ((t + j * F::M) >> 1) * n + at0);
     F::load_tw1(w1, a.tw_m, t);
 #pragma unroll
     for (int j = 0; j < F::R1; ++j) v[j] = swap(v[j]);
@@ -615,7 +617,7 @@ struct RowsInvP {
     int field_stride;   // elements between neighbouring bins of a field: 2 when interleaved
     const DevState * st;
 };
-template <int N, int P>
+template <int N, int P, bool INNER = false>
 __device__ __forceinline__ void rows_inv_body(const RowsInvP &a, int bid, int nblk) {
     using F = PairFft<N, P>;
     if (a.st && a.st->done) return;
@@ -635,8 +637,8 @@ __device__ __forceinline__ void rows_inv_body(const RowsInvP &a, int bid, int nb
 #pragma unroll
     for (int j = 0; j < F::R1; ++j) {
         const int u = t + j * F::M, un = (N - u) & (N - 1);
-        v[j] = F::load(in + (sine ? un : u));
-        xn[j] = F::load(in + (sine ? u : un));
+        v[j] = F::template load_pair<INNER>(in + (sine ? un : u));
+        xn[j] = F::template load_pair<INNER>(in + (sine ? u : un));
     }
 #pragma unroll
     for (int j = 0; j < F::R1; ++j) ek[j] = F::load(a.ek_n + t + j * F::M);
@@ -673,6 +675,44 @@ __device__ __forceinline__ void rows_inv_body(const RowsInvP &a, int bid, int nb
 template <int N, int P>
 __global__ void __launch_bounds__(PairFft<N, P>::THREADS) k_rows_inv(const __grid_constant__ RowsInvP p) {
     rows_inv_body<N, P>(p, blockIdx.x, gridDim.x);
+}
+
+// The isolated solve of a small grid (both sides 64 or 128) as one launch of one
+// cluster: the three passes with cluster barriers between them, each pass's blocks
+// dealt out to the CTAs.  Its bound is latency: 16 KB to 64 KB per array, and of three
+// launches back to back each took 4 to 5 us where its kernel works for about 2.
+// Per solve, three launches and this (us): 64 x 64 13.3, 8.2; 64 x 128 14.3, 10.2;
+// 128 x 64 15.4, 12.0; 128 x 128 16.4, 12.3; with the potential 14.3, 10.2 and 16.4,
+// 14.3 at the ends.  CTAs x pairs per block at 64 x 64: 8 x 8 and 8 x 4 8.2, 4 x 8
+// 10.2, 8 x 2 and 2 x 16 12.3, 1 x 16 18.4; at 128 x 128 8 x 8 12.3, 8 x 4 16.4,
+// 4 x 16 20.5.  Not for 256 x 256 (16.4, 31.6 this way: eight SMs are too few) and not
+// in the step, where the graph's launches cost less than the barriers (a pass of 8
+// steps at 64 x 64 bins 347, 350 with this).
+constexpr int kSmallCtas = 8, kSmallPairs = 8;
+struct SmallP {
+    RowsFwdP fwd;
+    ColsP cols;
+    RowsInvP inv;
+};
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <int M, int N>
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(PairFft<N, kSmallPairs>::THREADS)
+    k_solve_small(const __grid_constant__ SmallP p) {
+    constexpr int P = kSmallPairs, ROWS = M / (2 * P), COLS = N / (2 * P);
+    static_assert(PairFft<N, P>::THREADS == PairFft<M, P>::THREADS, "one block shape for all passes");
+    static_assert(ROWS <= kSmallCtas && COLS <= kSmallCtas, "at most one block per CTA");
+    const int cta = blockIdx.x;
+    if (cta < ROWS) rows_fwd_body<N, P>(p.fwd, cta, ROWS);
+    cluster_barrier();
+    if (cta < COLS) cols_body<M, P, true>(p.cols, cta, COLS);
+    cluster_barrier();
+    const int blocks = M / P + (p.inv.psi ? M / (2 * P) : 0);
+    for (int b = cta; b < blocks; b += kSmallCtas) {
+        rows_inv_body<N, P, true>(p.inv, b, blocks);
+        __syncthreads();   // the exchange area is free for the next block
+    }
 }
 
 // The density map as rho for the tensor-core solve: the conversion of R1 (same
@@ -897,6 +937,19 @@ struct LaunchRowsInv {
     }
 };
 
+static bool small_grid(int m, int n) { return (m == 64 || m == 128) && (n == 64 || n == 128); }
+template <int M, int N>
+static void launch_small_as(const SpectralPlan &p, const SpectralArgs &a) {
+    constexpr int P = kSmallPairs;
+    const size_t smem = std::max(rows_fwd_smem<N, P>(false), std::max(cols_pair_smem<M, P>(), rows_inv_smem<N, P>()));
+    k_solve_small<M, N><<<kSmallCtas, PairFft<N, P>::THREADS, smem, p.stream>>>(
+        SmallP{LaunchRowsFwd::params(p, a), LaunchCols::params(p, a), LaunchRowsInv::params(p, a)});
+}
+static void launch_small(const SpectralPlan &p, const SpectralArgs &a) {
+    if (p.m == 64) (p.n == 64 ? launch_small_as<64, 64> : launch_small_as<64, 128>)(p, a);
+    else (p.n == 64 ? launch_small_as<128, 64> : launch_small_as<128, 128>)(p, a);
+}
+
 // Opt the spectral kernels into large dynamic shared memory on the current device.
 struct PrepareRowsFwd {
     cudaError_t &e;
@@ -941,6 +994,7 @@ void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a) {
     const int m = p.m, n = p.n;
     const bool from_map = a.rho_in == nullptr;
     const int rb = m / (2 * kRowPairs);
+    if (small_grid(m, n) && !from_map) return launch_small(p, a);   // an isolated solve
     if (pair_side(n)) {
         pair_dispatch<PASS_ROWS_FWD>(n, p.seqs, LaunchRowsFwd{p, a});
     } else {

@@ -35,6 +35,30 @@ def test_solve_buffers(m, n):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("m,n", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_small_grid_in_one_launch(m, n):
+    """An isolated solve of a small grid is one launch of a cluster, a placement's is
+    three launches: the same density gives the same bits, with and without the
+    potential, twice in a row on the same intermediates."""
+    import torch
+    import reda_erplacer_gb300 as R
+    from designs import small_synth
+    p = R.Placement(small_synth(900, seed=m + 2 * n, macros=2), (m, n), 1.0, start_mode=1)
+    p.compute_potential(0)
+    rho, want = p.array("DENSITY"), [p.array(k) for k in ("FIELD_X", "FIELD_Y", "POTENTIAL")]
+    info = p.scalars()
+    p.close()
+    src = torch.from_numpy(np.ascontiguousarray(rho)).cuda()
+    s = R.SpectralSolver(m, n, info["bin_w"], info["bin_h"], stream=torch.cuda.current_stream().cuda_stream)
+    for psi in (True, False, True):
+        out = [torch.zeros(m * n, dtype=torch.float32, device="cuda") for _ in range(3)]
+        s.solve(src.data_ptr(), out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr() if psi else None)
+        torch.cuda.synchronize()
+        for got, ref in list(zip(out, want))[:3 if psi else 2]:
+            assert np.array_equal(got.cpu().numpy(), ref.reshape(-1))
+    s.close()
+
+
 @pytest.mark.parametrize("precision", [1, 2])
 @pytest.mark.parametrize("m,n", [(128, 128), (128, 2048), (2048, 128), (256, 512), (1024, 1024), (2048, 2048)])
 def test_contraction_tiles(m, n, precision):
