@@ -1,6 +1,7 @@
 // C ABI of liberplacer_gb300.so (include/erplacer.h): context set-up
 // (Placement::new, src/placement.rs:159-178), the reference's stage entry
 // points, the CUDA-graph Placement::step, the run loop and accessors.
+#include <limits.h>
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -964,8 +965,14 @@ extern "C" erp_status erp_set_scalars(erp_ctx *ctx, int32_t iteration, float gam
 extern "C" erp_status erp_get_positions(erp_ctx *ctx, float *x, float *y) {
     CTX_CHECK();
     if (!x || !y) return ERP_EINVAL;
-    CK(cudaMemcpyAsync(x, c.x, sizeof(float) * c.N, cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaMemcpyAsync(y, c.y, sizeof(float) * c.N, cudaMemcpyDeviceToHost, c.stream));
+    float *dx = mapped_host(x, c.N), *dy = mapped_host(y, c.N);
+    if (dx && dy) {
+        launch_xy_to_host(c, dx, dy);
+        CK(cudaGetLastError());
+    } else {
+        CK(cudaMemcpyAsync(x, c.x, sizeof(float) * c.N, cudaMemcpyDeviceToHost, c.stream));
+        CK(cudaMemcpyAsync(y, c.y, sizeof(float) * c.N, cudaMemcpyDeviceToHost, c.stream));
+    }
     CK(cudaStreamSynchronize(c.stream));
     return ERP_OK;
 }
@@ -1275,6 +1282,13 @@ extern "C" erp_status erp_checkpoint(erp_ctx *ctx, void *buf, size_t bytes) {
     return ERP_OK;
 }
 
+// The device address of a checkpoint's arrays where the buffer is device-mapped and
+// they lie on float boundaries, else nullptr (the arrays are copied).
+static const float *mapped_checkpoint(const char *arrays, int n) {
+    if ((reinterpret_cast<uintptr_t>(arrays) & 3) || n > INT_MAX / kCkptArrays) return nullptr;
+    return mapped_host(reinterpret_cast<float *>(const_cast<char *>(arrays)), n * kCkptArrays);
+}
+
 extern "C" erp_status erp_restore(erp_ctx *ctx, const void *buf, size_t bytes) {
     CTX_CHECK();
     if (!buf || bytes < sizeof(CkptHeader)) { c.err = "not a checkpoint"; return ERP_EINVAL; }
@@ -1295,14 +1309,18 @@ extern "C" erp_status erp_restore(erp_ctx *ctx, const void *buf, size_t bytes) {
     // must not leave the last-block finalizes of the next step unreachable
     memset(c.h_st->ctr, 0, sizeof c.h_st->ctr);
     c.h_st->expire_waits = c.expire_waits;   // the restoring context's own wait rule
-    CK(cudaMemcpyAsync(c.st, c.h_st, sizeof(DevState), cudaMemcpyHostToDevice, c.stream));
     i += sizeof(DevState);
-    float *arr[kCkptArrays] = {c.x, c.y, c.prev_x, c.prev_y, c.prev_gx, c.prev_gy};
-    for (float *a : arr) {
-        CK(cudaMemcpyAsync(a, i, sizeof(float) * c.N, cudaMemcpyHostToDevice, c.stream));
-        i += sizeof(float) * c.N;
+    if (const float *src = mapped_checkpoint(i, c.N)) {
+        launch_restore(c, src, *c.h_st);
+    } else {
+        CK(cudaMemcpyAsync(c.st, c.h_st, sizeof(DevState), cudaMemcpyHostToDevice, c.stream));
+        float *arr[kCkptArrays] = {c.x, c.y, c.prev_x, c.prev_y, c.prev_gx, c.prev_gy};
+        for (float *a : arr) {
+            CK(cudaMemcpyAsync(a, i, sizeof(float) * c.N, cudaMemcpyHostToDevice, c.stream));
+            i += sizeof(float) * c.N;
+        }
+        launch_pack_xy(c);
     }
-    launch_pack_xy(c);
     c.map_dirty = true;   // the next step starts from a cleared map
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c.stream));

@@ -175,6 +175,7 @@ void launch_scatter_items(Ctx &c, cudaStream_t s);   // its work items again, af
 int scatter_tiles(int m, int n);
 int scatter_items_max(int NM, int m, int n);
 void launch_xy_from_host(Ctx &c, const float *hx, const float *hy);   // device-mapped host x, y -> x, y, xy
+void launch_restore(Ctx &c, const float *src, const DevState &state);   // a checkpoint's arrays in device-mapped host memory
 void launch_xy_to_host(Ctx &c, float *hx, float *hy);                 // xy -> device-mapped host x, y
 cudaError_t place_occupancy();                        // resident block counts of the streaming kernels
 constexpr int kSortEvery = 16;                          // steps between scatter-order refreshes

@@ -1,0 +1,53 @@
+"""Checkpoints and positions in device-mapped (pinned) host memory are read and
+written by kernels, other memory by copies: the same state and the same bits
+either way, on every alignment of the buffers and for every remainder of four
+cells, with nothing written outside the arrays."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from designs import small_synth
+
+pytestmark = pytest.mark.gpu
+
+F32P = C.POINTER(C.c_float)
+
+
+def pinned(nbytes):
+    import torch
+    return torch.empty(nbytes, dtype=torch.uint8, pin_memory=True).numpy()
+
+
+@pytest.mark.parametrize("cells", [900, 901, 902, 903, 5])
+def test_mapped_and_other_memory_agree(cells):
+    import reda_erplacer_gb300 as R
+    p = R.Placement(small_synth(cells, seed=9, macros=2, io=30), (64, 64), 1.0, start_mode=1)
+    p.run(3)
+    blob = np.frombuffer(p.checkpoint(), np.uint8)
+    start = [a.copy() for a in p.positions()]
+    p.run(4)
+    want = [a.copy() for a in p.positions()] + [p.array("PREV_X"), p.scalars()]
+    for shift in (None, 0, 4, 8, 12, 1, 2):   # ordinary memory; pinned, on a boundary of floats or not
+        if shift is None:
+            at = blob.copy()
+        else:
+            at = pinned(blob.nbytes + 16)[shift:shift + blob.nbytes]
+            at[:] = blob
+        assert p.lib.erp_restore(p.h, at.ctypes.data, at.nbytes) == 0
+        for a, b in zip(p.positions(), start):
+            assert np.array_equal(a, b)
+        p.run(4)
+        for a, b in zip(p.positions(), want):
+            assert np.array_equal(a, b)
+        assert np.array_equal(p.array("PREV_X"), want[2]) and p.scalars() == want[3]
+    n = p.N
+    for ox, oy in ((0, 0), (1, 0), (0, 1), (1, 3)):
+        x, y = (pinned(4 * (n + 8)).view(np.float32) for _ in range(2))
+        x[:] = y[:] = -7.0
+        u, v = x[ox:ox + n], y[oy:oy + n]
+        assert p.lib.erp_get_positions(p.h, u.ctypes.data_as(F32P), v.ctypes.data_as(F32P)) == 0
+        assert np.array_equal(u, want[0]) and np.array_equal(v, want[1])
+        for buf, o in ((x, ox), (y, oy)):
+            assert (buf[:o] == -7.0).all() and (buf[o + n:] == -7.0).all()
+    p.close()
