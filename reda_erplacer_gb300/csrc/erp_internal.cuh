@@ -187,6 +187,11 @@ void launch_scheduler(Ctx &c, int use_args, float hpwl, float overflow);
 // One whole Placement::step on the context's stream (the graph's content); with a
 // second stream and two events, under capture, in two branches up to the force.
 void enqueue_step_kernels(Ctx &c, cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+// Several contexts' states to their page-locked host copies (hosts[i], device
+// addresses), or the stop rule of their next steps set.
+void launch_pull_states(DevState *const *states, DevState *const *hosts, int count, cudaStream_t s);
+void launch_arm_states(DevState *const *states, int count, float stop_overflow, int max_iterations, cudaStream_t s);
+void launch_disarm_states(DevState *const *states, int count, cudaStream_t s);
 // Gather the retire flags of several contexts into out[i] (device pointers).
 void launch_gather_done(DevState *const *states, int count, int32_t *out, cudaStream_t s);
 

@@ -1457,6 +1457,33 @@ __global__ void k_gather_done(DevState *const *states, int count, int32_t *out) 
         out[i] = states[i]->done;
 }
 
+// A block per context: its state to the host, one word per thread.  32 contexts: one
+// launch for 32 copies and 32 waits, before and after every batched run.
+__global__ void __launch_bounds__(kThreads) k_pull_states(DevState *const *states, DevState *const *hosts) {
+    static_assert(sizeof(DevState) % 4 == 0 && sizeof(DevState) / 4 <= kThreads, "one word per thread");
+    if (threadIdx.x < sizeof(DevState) / 4)
+        reinterpret_cast<uint32_t *>(hosts[blockIdx.x])[threadIdx.x] =
+            reinterpret_cast<const uint32_t *>(states[blockIdx.x])[threadIdx.x];
+}
+
+// Retire at the overflow or after max_iterations more steps; max_iterations < 0: never.
+__global__ void k_arm_states(DevState *const *states, int count, float stop_overflow, int max_iterations) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        DevState *st = states[i];
+        st->stop_overflow = max_iterations >= 0 && stop_overflow > 0 ? stop_overflow : 0.0f;
+        st->stop_iter = max_iterations >= 0 ? st->iteration + max_iterations : 0;
+        st->done = max_iterations == 0 ? 1 : 0;
+    }
+}
+
+void launch_pull_states(DevState *const *states, DevState *const *hosts, int count, cudaStream_t s) {
+    if (count > 0) k_pull_states<<<count, kThreads, 0, s>>>(states, hosts);
+}
+void launch_arm_states(DevState *const *states, int count, float stop_overflow, int max_iterations, cudaStream_t s) {
+    k_arm_states<<<(count + 255) / 256, 256, 0, s>>>(states, count, stop_overflow, max_iterations);
+}
+void launch_disarm_states(DevState *const *states, int count, cudaStream_t s) { launch_arm_states(states, count, 0.0f, -1, s); }
+
 void launch_gather_done(DevState *const *states, int count, int32_t *out, cudaStream_t s) {
     k_gather_done<<<(count + 255) / 256, 256, 0, s>>>(states, count, out);
 }
@@ -1712,7 +1739,6 @@ struct RestoreP {
     DevState *st;
 };
 __global__ void __launch_bounds__(kThreads) k_restore(const __grid_constant__ RestoreP p) {
-    static_assert(sizeof(DevState) % 4 == 0 && sizeof(DevState) / 4 <= kThreads, "one word per thread");
     if (blockIdx.x == 0 && threadIdx.x < sizeof(DevState) / 4)
         reinterpret_cast<uint32_t *>(p.st)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&p.state)[threadIdx.x];
     const size_t N = (size_t)p.N;
