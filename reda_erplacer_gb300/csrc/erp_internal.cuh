@@ -56,9 +56,11 @@ struct DevState {
 
 constexpr int32_t kStatusWaitTimeout = 2;   // DevState::status bit 1
 
-// ctr[CTR_UPDATE] is a flag, not a counter: the current step's position update is due
-// (set by k_nesterov_grad, cleared by the step's first kernel).
-enum Counter { CTR_HPWL = 0, CTR_OVF = 1, CTR_ABS = 2, CTR_LIP = 3, CTR_ENERGY = 4, CTR_UPDATE = 7 };
+// The last three are no counters.  ctr[CTR_UPDATE]: the current step's position update
+// is due (set by k_nesterov_grad, cleared by the step's first kernel); CTR_ALPHA and
+// CTR_ITER: alpha's bits and the iteration as the update has to see them in every block
+// while one of them writes the next (set by k_nesterov_grad).
+enum Counter { CTR_HPWL = 0, CTR_OVF = 1, CTR_ABS = 2, CTR_ENERGY = 4, CTR_ALPHA = 5, CTR_ITER = 6, CTR_UPDATE = 7 };
 
 // Net degree classes processed by one thread group of width W each.
 // Classes 0..7 hold nets of one exact degree -- class 0 the leading 2-pin nets

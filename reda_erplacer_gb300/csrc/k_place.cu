@@ -1080,9 +1080,8 @@ __global__ void __launch_bounds__(kThreads) k_dw_rescale(int NM, int iter_arg,
 
 // Preconditioned combined gradient and Lipschitz sums (src/nesterov.rs:74-95);
 // the gradient replaces prev_g (the reference copies it there after the update,
-// src/nesterov.rs:143-144, and nothing reads prev_g in between).  The last block
-// applies update_momentum (src/nesterov.rs:148-158) and the adaptive step
-// length (src/nesterov.rs:98-100).
+// src/nesterov.rs:143-144, and nothing reads prev_g in between).  The block sums
+// are left for the update, which takes the step length from them.
 //
 // Both Nesterov kernels move four cells per thread with 128-bit loads and
 // stores (the per-cell arrays are 256-byte aligned; a scalar tail covers
@@ -1190,25 +1189,41 @@ __device__ __forceinline__ void nesterov_grad_body(const GradP &p, int bid, int 
     }
     Df vals[2] = {Df{numf, 0.0f}, Df{denf, 0.0f}};
     block_sums(vals, shr);
-    if (!arrive_last(partials, bid, 2, vals, &st->ctr[CTR_LIP], nblk)) return;
-    Df tot[2] = {partials_share(partials, nblk, 2, 0), partials_share(partials, nblk, 2, 1)};
-    block_sums(tot, shr);
-    if (threadIdx.x == 0) {
-        const double tn = df_value(tot[0]), td = df_value(tot[1]);
-        // update_momentum (src/nesterov.rs:148-158), adaptive step length (:98-100)
-        const int it = iter_arg >= 0 ? iter_arg : st->iteration;
-        const float one = 1.0f, two = one + one, four = two + two;
-        const float a_prev = st->alpha;
-        const float na = (one + sqrtf(four * a_prev * a_prev + one)) / two;
-        st->beta = (a_prev - one) / na;
-        st->alpha = it > 0 && td > 0.0 ? (float)sqrt(tn / td) : na;
-        st->lip_num = tn;
-        st->lip_den = td;
-        if (p.step) st->ctr[CTR_UPDATE] = 1;
-        st->ctr[CTR_LIP] = 0;
+    if (threadIdx.x == 0) {   // for the update (nesterov_alpha)
+        Df *part = reinterpret_cast<Df *>(partials) + 2 * (size_t)bid;
+        part[0] = vals[0];
+        part[1] = vals[1];
+        if (bid == 0) {
+            st->ctr[CTR_ALPHA] = __float_as_uint(st->alpha);
+            st->ctr[CTR_ITER] = (uint32_t)(iter_arg >= 0 ? iter_arg : st->iteration);
+            if (p.step) st->ctr[CTR_UPDATE] = 1;
+        }
     }
 }
 __global__ void __launch_bounds__(kThreads) k_nesterov_grad(const __grid_constant__ GradP p) { nesterov_grad_body(p, blockIdx.x, gridDim.x); }
+
+// The step's alpha and beta from the sums of k_nesterov_grad's block sums, which every
+// block of the update adds up for itself: update_momentum (src/nesterov.rs:148-158) and
+// the adaptive step length (:98-100).  By the gradient pass's last block it took a
+// fence, an arrival counter, a second fence and the sums read back, one after another:
+// 5.3 us of gradient pass and 4.3 of update at 2,000 cells, now 2.8 and 5.3 (the step's
+// tail in block 0 is the longest); 15.5 and 9.6 at 1M, now 12.4 and 11.5.  A pass of
+// restore, steps and positions at 2,000 cells 319 -> 305 us, at 20,000 302 -> 291, at
+// 200,000 371 -> 365.
+__device__ __forceinline__ void nesterov_alpha(double num, double den, float a_prev, int it, float *ab) {
+    const float one = 1.0f, two = one + one, four = two + two;
+    const float na = (one + sqrtf(four * a_prev * a_prev + one)) / two;
+    ab[0] = it > 0 && den > 0.0 ? (float)sqrt(num / den) : na;
+    ab[1] = (a_prev - one) / na;
+}
+__device__ __forceinline__ void leave_alpha(DevState *st, double num, double den, const float *ab) {
+    st->alpha = ab[0];
+    st->beta = ab[1];
+    st->lip_num = num;
+    st->lip_den = den;
+}
+// warps 0 and 1 of a block
+__device__ __forceinline__ void alpha_barrier() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
 
 
 // ============================ scheduler ============================
@@ -1220,11 +1235,21 @@ struct SchedLogs {
 // step record, the non-finite check and the retire-at-overflow flag; one warp, all
 // lanes with the same totals.  The state is loaded up front, so that its latencies
 // overlap the arithmetic.
-__device__ __forceinline__ void run_scheduler(DevState *st, const SchedLogs &lg, float hpwl, float ovf) {
+struct SchedIn {
+    int it, init_set, ovf_set, stop_iter;
+    float init, prev, ovf_prev, dw, gamma, base_gamma, stop_overflow;
+};
+__device__ __forceinline__ SchedIn sched_in(const DevState *st) {
+    return SchedIn{st->iteration, st->hpwl_init_set, st->ovf_init_set, st->stop_iter, st->hpwl_init, st->hpwl_cur,
+                   st->ovf_cur, st->dw, st->gamma, st->base_gamma, st->stop_overflow};
+}
+template <bool IN_STEP>
+__device__ __forceinline__ void run_scheduler(DevState *st, const SchedIn &in, const SchedLogs &lg, float hpwl, float ovf,
+                                              const float *ab) {
     const int lane = threadIdx.x & 31;
-    const int it = st->iteration, init_set = st->hpwl_init_set, ovf_set = st->ovf_init_set, stop_iter = st->stop_iter;
-    const float init = st->hpwl_init, prev = st->hpwl_cur, ovf_prev = st->ovf_cur, dw = st->dw, gamma = st->gamma;
-    const float base_gamma = st->base_gamma, alpha = st->alpha, beta = st->beta, stop_overflow = st->stop_overflow;
+    const int it = in.it, init_set = in.init_set, ovf_set = in.ovf_set, stop_iter = in.stop_iter;
+    const float init = in.init, prev = in.prev, ovf_prev = in.ovf_prev, dw = in.dw, gamma = in.gamma;
+    const float base_gamma = in.base_gamma, stop_overflow = in.stop_overflow;
     // The density-weight power (lane 0) and the gamma coefficient (lane 1) are
     // independent FP64 powers of constant bases, b^e = exp(e ln b) with ln b
     // computed on the host: one convergent exp call evaluates both.  (FP64 runs
@@ -1256,7 +1281,9 @@ __device__ __forceinline__ void run_scheduler(DevState *st, const SchedLogs &lg,
     else if (delta0 < 0.0f) pw = pw < 0.98 ? 0.98 : pw;
     else pw = pw < 0.95 ? 0.95 : (pw > 1.05 ? 1.05 : pw);
     const double coef_l1 = __shfl_sync(0xffffffffu, pw, 1);
+    if (IN_STEP) alpha_barrier();
     if (lane != 0) return;
+    const float alpha = ab[0], beta = ab[1];
     erp_step_stats rec;
     rec.iteration = it;
     rec.should_stop = (prev != 0.0f && hpwl != 0.0f && prev > hpwl * 1.5f) ? 1 : 0;
@@ -1293,19 +1320,21 @@ struct SchedP {
 __global__ void k_scheduler(const __grid_constant__ SchedP p) {
     DevState *st = p.st;
     if (st->done) return;   // warp-uniform
-    run_scheduler(st, p.lg, p.use_args ? p.hpwl_arg : st->hpwl_f, p.use_args ? p.ovf_arg : st->overflow_f);
+    const float ab[2] = {st->alpha, st->beta};
+    run_scheduler<false>(st, sched_in(st), p.lg, p.use_args ? p.hpwl_arg : st->hpwl_f, p.use_args ? p.ovf_arg : st->overflow_f, ab);
 }
 
 // Block 0 of a whole step's position update: the HPWL and overflow totals, from the
-// block sums that k_wa and the map conversion left, and the scheduler.  Nothing of
-// the step needs them earlier, and the update's blocks beside it read only alpha,
-// beta and ctr[CTR_UPDATE] (the scheduler may set `done`, with which the update must
-// still run).  A reduction's own tail -- arrival counter, fences, last block's sum --
-// cost 2 to 3 us of kernels that take 3 to 5 at 2,000 cells, and the scheduler's
-// launch 3.3 us; here both hide behind the update.  A step takes 5.6 us less at 2,000
-// and 20,000 cells, 7 us at 200,000 and 8 us at 1M.  (Run by k_nesterov_grad's last
-// block instead, the tail was serial: 9.0 us of gradient pass at 20,000 cells, 5.4 us
-// this way.)
+// block sums that k_wa and the map conversion left, the step length for the record
+// (warp 1, beside the scheduler's powers in warp 0), and the scheduler.  Nothing of the
+// step needs them earlier, and the update's blocks beside it read nothing that this one
+// writes (CTR_ALPHA and CTR_ITER are copies; the scheduler may set `done`, with which
+// the update must still run).  A reduction's own tail -- arrival counter, fences, last
+// block's sum -- cost 2 to 3 us of kernels that take 3 to 5 at 2,000 cells, and the
+// scheduler's launch 3.3 us; here both hide behind the update.  A step takes 5.6 us less
+// at 2,000 and 20,000 cells, 7 us at 200,000 and 8 us at 1M.  (Run by k_nesterov_grad's
+// last block instead, the tail was serial: 9.0 us of gradient pass at 20,000 cells.)
+// The state that the scheduler reads is loaded with the sums: 5.7 us, 5.3 this way.
 struct StepTailP {
     int n_wl, n_ovf;   // block sums of the HPWL and of the overflow
     const double * part_wl;
@@ -1313,23 +1342,37 @@ struct StepTailP {
     double movable_area;
     SchedLogs lg;
 };
-__device__ __forceinline__ void step_tail(const StepTailP &p, DevState *st) {
-    __shared__ double shr[2 * (kThreads / 32)];
-    Df tot[2] = {partials_share(p.part_wl, p.n_wl, 1, 0), partials_share(p.part_ovf, p.n_ovf, 1, 0)};
+__device__ __forceinline__ void step_tail(const StepTailP &p, const double *lip, int n_lip, DevState *st) {
+    __shared__ double shr[4 * (kThreads / 32)], sum[4];
+    __shared__ float ab[2];
+    const float a_prev = __uint_as_float(st->ctr[CTR_ALPHA]);
+    const int it = (int)st->ctr[CTR_ITER];
+    const bool off = st->ctr[CTR_UPDATE] == 0;
+    const SchedIn in = sched_in(st);   // on the way with the sums
+    Df tot[4] = {partials_share(p.part_wl, p.n_wl, 1, 0), partials_share(p.part_ovf, p.n_ovf, 1, 0),
+                 partials_share(lip, n_lip, 2, 0), partials_share(lip, n_lip, 2, 1)};
     block_sums(tot, shr);
-    if (threadIdx.x >= 32) return;
-    double v[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        v[k] = df_value(Df{__shfl_sync(0xffffffffu, tot[k].hi, 0), __shfl_sync(0xffffffffu, tot[k].lo, 0)});
-    const float hpwl = (float)v[0], ovf = (float)(v[1] / p.movable_area);
-    if (threadIdx.x == 0) {
-        st->hpwl = v[0];
-        st->hpwl_f = hpwl;
-        st->overflow = v[1];
-        st->overflow_f = ovf;
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 4; ++k) sum[k] = df_value(tot[k]);
+    __syncthreads();
+    if (off) return;
+    const int warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const float hpwl = (float)sum[0], ovf = (float)(sum[1] / p.movable_area);
+        if (threadIdx.x == 0) {
+            st->hpwl = sum[0];
+            st->hpwl_f = hpwl;
+            st->overflow = sum[1];
+            st->overflow_f = ovf;
+        }
+        run_scheduler<true>(st, in, p.lg, hpwl, ovf, ab);
+    } else if (warp == 1) {   // beside the scheduler's powers
+        if (threadIdx.x == 32) {
+            nesterov_alpha(sum[2], sum[3], a_prev, it, ab);
+            leave_alpha(st, sum[2], sum[3], ab);
+        }
+        alpha_barrier();
     }
-    run_scheduler(st, p.lg, hpwl, ovf);
 }
 
 // ============================ position update ============================
@@ -1365,7 +1408,9 @@ struct UpdateP {
     const float * gy;
     float2 * xy;
     DevState * st;
-    int step;        // 1: inside a whole step: block 0 runs its tail
+    const double * lip;   // k_nesterov_grad's block sums
+    int n_lip;
+    int step;             // 1: inside a whole step: block 0 runs its tail
     StepTailP tail;
 };
 __device__ __forceinline__ void nesterov_update_body(const UpdateP &p, int bid, int nblk) {
@@ -1382,22 +1427,36 @@ __device__ __forceinline__ void nesterov_update_body(const UpdateP &p, int bid, 
     const float *__restrict__ gy = p.gy;
     float2 *__restrict__ xy = p.xy;
     DevState *st = p.st;
-    if (p.step) {
-        if (st->ctr[CTR_UPDATE] == 0) return;
-        if (bid == 0) {
-            step_tail(p.tail, st);
-            return;
-        }
-        --bid;
-        --nblk;
-    } else if (st->done) {
+    if (p.step && bid == 0) {
+        step_tail(p.tail, p.lip, p.n_lip, st);
         return;
     }
-    const float alpha = st->alpha, beta = st->beta;
-    const int n4 = NM >> 2;
-    for (int i4 = bid * blockDim.x + threadIdx.x; i4 < n4; i4 += nblk * blockDim.x) {
-        Cell4 xx = ld4w(x, i4), yy = ld4w(y, i4), qx = ld4w(px, i4), qy = ld4w(py, i4);
-        const Cell4 a = ld4(gx, i4), b = ld4(gy, i4), ww = ld4(w, i4), hh = ld4(h, i4);
+    const bool off = p.step ? st->ctr[CTR_UPDATE] == 0 : st->done;
+    // the flag, the first cells and the block sums are loaded together
+    __shared__ double shr[2 * (kThreads / 32)];
+    __shared__ float ab[2];
+    const int first = p.step ? 1 : 0, n4 = NM >> 2;
+    const int at = (bid - first) * (int)blockDim.x + (int)threadIdx.x, stride = (nblk - first) * (int)blockDim.x;
+    const float a_prev = __uint_as_float(st->ctr[CTR_ALPHA]);
+    const int it = (int)st->ctr[CTR_ITER];
+    Cell4 xx{}, yy{}, qx{}, qy{}, a{}, b{}, ww{}, hh{};
+    auto load = [&](int i4) {
+        xx = ld4w(x, i4), yy = ld4w(y, i4), qx = ld4w(px, i4), qy = ld4w(py, i4);
+        a = ld4(gx, i4), b = ld4(gy, i4), ww = ld4(w, i4), hh = ld4(h, i4);
+    };
+    if (at < n4) load(at);
+    Df tot[2] = {partials_share(p.lip, p.n_lip, 2, 0), partials_share(p.lip, p.n_lip, 2, 1)};
+    block_sums(tot, shr);
+    if (threadIdx.x == 0) {
+        const double num = df_value(tot[0]), den = df_value(tot[1]);
+        nesterov_alpha(num, den, a_prev, it, ab);
+        if (!p.step && bid == 0 && !off) leave_alpha(st, num, den, ab);
+    }
+    __syncthreads();
+    if (off) return;
+    const float alpha = ab[0], beta = ab[1];
+    for (int i4 = at; i4 < n4; i4 += stride) {
+        if (i4 != at) load(i4);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             nesterov_update_cell(xx.v[k], yy.v[k], qx.v[k], qy.v[k], a.v[k], b.v[k], ww.v[k], hh.v[k], die_w,
@@ -1410,8 +1469,8 @@ __device__ __forceinline__ void nesterov_update_body(const UpdateP &p, int bid, 
         xy4[0] = make_float4(xx.v[0], yy.v[0], xx.v[1], yy.v[1]);
         xy4[1] = make_float4(xx.v[2], yy.v[2], xx.v[3], yy.v[3]);
     }
-    if (bid == 0 && threadIdx.x < (NM & 3)) {
-        const int i = (n4 << 2) + threadIdx.x;
+    if (at < (NM & 3)) {
+        const int i = (n4 << 2) + at;
         float xi = x[i], yi = y[i], pxi = px[i], pyi = py[i];
         nesterov_update_cell(xi, yi, pxi, pyi, gx[i], gy[i], w[i], h[i], die_w, die_h, alpha, beta);
         x[i] = xi;
@@ -1674,10 +1733,11 @@ static SchedLogs sched_logs() {
     return lg;
 }
 
+static int lip_blocks(const Ctx &c) { return fit(grid_for((c.NM + 3) / 4), g_res_grad); }
 static int grad_params(Ctx &c, int iter_arg, bool step, GradP &p) {
     p = GradP{c.NM, iter_arg, c.wlgx, c.wlgy, c.dgp, c.pos, c.w, c.h, c.npins, c.x, c.y, c.prev_x, c.prev_y,
               c.prev_gx, c.prev_gy, c.partials, c.st, step ? 1 : 0};
-    return fit(grid_for((c.NM + 3) / 4), g_res_grad);
+    return lip_blocks(c);
 }
 
 static int update_params(Ctx &c, bool step, UpdateP &p) {
@@ -1688,7 +1748,7 @@ static int update_params(Ctx &c, bool step, UpdateP &p) {
                          sched_logs()};
     }
     p = UpdateP{c.NM, c.w, c.h, c.die_w, c.die_h, c.x, c.y, c.prev_x, c.prev_y, c.prev_gx, c.prev_gy, c.xy, c.st,
-                step ? 1 : 0, tail};
+                c.partials, lip_blocks(c), step ? 1 : 0, tail};
     return fit(grid_for((c.NM + 3) / 4), g_res_update) + (step ? 1 : 0);
 }
 
