@@ -44,12 +44,12 @@ struct WaArgs {
 };
 
 template <int W, int P>
-__device__ __forceinline__ float wa_class(const WaArgs &a, int net_begin, int net_count, int general,
+__device__ __forceinline__ Df wa_class(const WaArgs &a, int net_begin, int net_count, int general,
                                           int cblock, int cgrid) {
     const int gl = threadIdx.x & (W - 1);
     constexpr int GPB = kThreads / W;
     const float inv_gamma = a.inv_gamma;
-    float hp_acc = 0.0f;
+    Df hp_acc = df_zero();
     for (int base = cblock * GPB; base < net_count; base += cgrid * GPB) {
         const int gid = base + (int)threadIdx.x / W;
         const bool active = gid < net_count;
@@ -164,7 +164,7 @@ __device__ __forceinline__ float wa_class(const WaArgs &a, int net_begin, int ne
         if (active && gl == 0) {
             const float hp = (mxx - mnx) + (mxy - mny);   // src/hpwl.rs:302
             a.net_hpwl[e] = hp;
-            hp_acc += hp;
+            hp_acc = df_add(hp_acc, hp);
         }
     }
     return hp_acc;
@@ -174,10 +174,10 @@ __device__ __forceinline__ float wa_class(const WaArgs &a, int net_begin, int ne
 // class's net g at slot0 + q * count + g): the slot reads and gradient writes of
 // a warp are coalesced and no net_ptr is read.  Same arithmetic as wa_class.
 template <int D>
-__device__ __forceinline__ float wa_exact(const WaArgs &a, int net_begin, int net_count, int slot0,
+__device__ __forceinline__ Df wa_exact(const WaArgs &a, int net_begin, int net_count, int slot0,
                                           int general, int cblock, int cgrid) {
     const float inv_gamma = a.inv_gamma;
-    float hp_acc = 0.0f;
+    Df hp_acc = df_zero();
     for (int g = cblock * kThreads + (int)threadIdx.x; g < net_count; g += cgrid * kThreads) {
         float px[D], py[D];
         float mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
@@ -239,7 +239,7 @@ __device__ __forceinline__ float wa_exact(const WaArgs &a, int net_begin, int ne
                             __fmaf_rn(__fmaf_rn(b_y, py[q], a_y), ey[q], -(__fmaf_rn(b_ny, py[q], a_ny) * eny[q])));
         const float hp = (mxx - mnx) + (mxy - mny);   // src/hpwl.rs:302
         a.net_hpwl[net_begin + g] = hp;
-        hp_acc += hp;
+        hp_acc = df_add(hp_acc, hp);
     }
     return hp_acc;
 }
@@ -277,7 +277,7 @@ __device__ __forceinline__ void wa_body(const WaP &p, int bid, int nblk) {
     int k = 0;
     while (k + 1 < kNumClasses && vb >= cl.block0[k + 1]) ++k;
     const int cb = vb - cl.block0[k], cg = cl.block0[k + 1] - cl.block0[k];
-    float hp;
+    Df hp;
 #define ERP_WA_EXACT(K, D) \
     case K: hp = wa_exact<D>(a, cl.begin[K], cl.count[K], cl.slot0[K], cl.general[K], cb, cg); break;
     switch (k) {
@@ -1553,6 +1553,8 @@ static int grid_for(int work, int cap = 152 * 8) {
     return g < 1 ? 1 : (g > cap ? cap : g);
 }
 
+constexpr int kWaBlocks = 152 * 4;   // k_wa's blocks that are resident at once
+static_assert(kWaBlocks <= kMaxPartials, "a block sum per block");
 static int wa_params(Ctx &c, float gamma_arg, bool step, WaP &p) {
     WaArgs a;
     a.net_ptr = c.net_ptr;
@@ -1565,15 +1567,29 @@ static int wa_params(Ctx &c, float gamma_arg, bool step, WaP &p) {
     a.def_min_x = c.die_w + 1.0f;
     a.def_min_y = c.die_h + 1.0f;
     WaClasses cl;
-    // at most 256 blocks per class: grid-stride loops over several nets per
-    // thread measured fastest on the 1M-cell workload (256: 93 us, 1024: 107 us,
-    // one net per thread: 121 us); fewer if the block partials of the HPWL sum
-    // would not fit, then every class's grid shrinks in proportion
-    long long need[kNumClasses], total = 0;
+    // One net per thread while that fits into kWaBlocks blocks; beyond, every class's
+    // threads take as many nets as fit into one common time, a net costing about its
+    // pins and one more (a lane group's nets 9, or 6 for a whole warp's).  So the blocks
+    // are resident at once and end together: with at most 256 blocks per class, an SM
+    // idled a quarter of the time at 1M cells.  k_wa at 1M 50.6 -> 45.2 us, 200,000
+    // cells 15.4 -> 13.4; with 1216 blocks 47.4 and 15.3, 2432 51.6, 3648 56; weights of
+    // the groups 6, 9, 14: 44.5, 45.2, 53 at 1M and 16.2, 13.4, 16.0 at 200,000.  (The
+    // next net's slots loaded a net ahead: no change.)  A pass of a few steps: 799 ->
+    // 790 us at 1M, 369.5 -> 366 at 200,000.  The nets of a thread add up their HPWL in
+    // double-float, so that their number costs no bits.
+    int need[kNumClasses], nets[kNumClasses];
     for (int k = 0; k < kNumClasses; ++k) {
         const int gpb = kThreads / c.cls[k].width;
-        need[k] = std::min<long long>((c.cls[k].count + gpb - 1) / gpb, 256);
-        total += need[k];
+        need[k] = (c.cls[k].count + gpb - 1) / gpb;
+    }
+    for (float time = 0.0f;; time = time * 1.05f + 1.0f) {
+        long long total = 0;
+        for (int k = 0; k < kNumClasses; ++k) {
+            const int cost = 1 + (c.cls[k].degree ? c.cls[k].degree : (c.cls[k].width == 32 ? 6 : 9));
+            nets[k] = std::max(1, (int)(time / (float)cost));
+            total += (need[k] + nets[k] - 1) / nets[k];
+        }
+        if (total <= kWaBlocks) break;
     }
     int blocks = 0;
     for (int k = 0; k < kNumClasses; ++k) {
@@ -1583,12 +1599,7 @@ static int wa_params(Ctx &c, float gamma_arg, bool step, WaP &p) {
         cl.general[k] = nc.general;
         cl.slot0[k] = nc.slot0;
         cl.block0[k] = blocks;
-        long long g = need[k];
-        if (total > c.max_partials && g > 0) {
-            g = need[k] * (c.max_partials - kNumClasses) / total;
-            if (g < 1) g = 1;
-        }
-        blocks += (int)g;
+        blocks += (need[k] + nets[k] - 1) / nets[k];
     }
     cl.block0[kNumClasses] = blocks;
     p = WaP{a, cl, gamma_arg, step ? 1 : 0, step ? c.part_wl : c.partials, c.st};
