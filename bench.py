@@ -363,12 +363,12 @@ def batch_section(args, device, world=1, rank=0):
             "tiny_mix_packed_jobs_per_hour": n_tiny / forms["tiny_mix_packed_s"] * 3600.0,
             "tiny_mix_branches_jobs_per_hour": n_tiny / forms["tiny_mix_branches_s"] * 3600.0,
             "note": "packed: the FP32 instances with bins <= 256 advance in one launch per stage over a table of "
-                    "all of them; branches: a graph branch of ten kernels per instance. Same bits either way; "
+                    "all of them; branches: a graph branch of nine kernels per instance. Same bits either way; "
                     "times include context creation"},
         "spectral_autotune": {"seqs_per_block": spec_chosen,
                               "candidates_ms": {str(c): round(t, 4) for c, t in spec_ms},
                               "note": "rows / columns per block of the FP32 passes at sides 64-256 (0 = the "
-                                      "fixed four); timed at creation, all FP32 instances' passes together; "
+                                      "fixed shape); timed at creation, all FP32 instances' passes together; "
                                       "included in batched_s"},
         "mixed_batched": {
             "spectral": "BF16 hi/lo x3 tensor-core contractions (bins >= 128), FP32 FFT (64^2 bins)",

@@ -1334,7 +1334,7 @@ struct erp_batch {
     cudaStream_t master = nullptr;
     int scatter_cells = 0;                 // autotuned cells per scatter block (0: the alone rule)
     std::vector<std::pair<int, float>> tuning;   // (candidate, ms of all instances' scatters together)
-    int spectral_seqs = 0;                 // autotuned sequences per block of the warp-form spectral passes
+    int spectral_seqs = 0;                 // autotuned sequences per block of the spectral passes
     bool packed = true;                    // small FP32 instances in packed launches (else a branch each)
     int packed_instances = 0;              // how many of them (at creation)
     void *pack_dev = nullptr;              // argument tables of the packed launches
@@ -1585,9 +1585,9 @@ static erp_status batch_tune_scatter(erp_batch *b) {
 }
 
 // Autotuner of the spectral passes' tile shape for a batch: the sequences (rows
-// or columns) per block of the warp-form passes, which serve the sides 64..256
-// that most instances of a mix have.  Alone, four per block measured fastest
-// at every side; with every instance's passes on the GPU at once the best shape
+// or columns) per block of the passes of sides 64..256, which most instances of a
+// mix have.  Alone, the fixed pairs per block (k_spectral.cu) measured fastest at
+// every side; with every instance's passes on the GPU at once the best shape
 // can differ, as for the scatter.  Each candidate is timed on a graph of all FP32
 // instances' three passes running together, and the fastest is kept.  The
 // passes read the (cleared) map and the fixed-cell map and write only the
@@ -1693,7 +1693,7 @@ extern "C" erp_status erp_batch_spectral_tuning(const erp_batch *b, int32_t *cho
 }
 
 // Whether an instance's step runs in the batch's packed launches: the FP32
-// solve in its warp forms (bins 64..256 on both axes), with movable cells and
+// solve (bins 64..256 on both axes), with movable cells and
 // nets, and at most 100,000 movable cells (ERP_BATCH_PACK_MAX_CELLS sets the
 // cap).  Larger grids, whose kernels are long enough for their launches not to
 // matter, and the tensor-core solve keep a graph branch each; so do the larger

@@ -121,7 +121,7 @@ struct Ctx {
     int32_t scatter_cells;     // movable cells per scatter item; 0: the rule for a context run alone
                                // (call launch_scatter_items after a change)
     int32_t scatter_bits;      // every contribution of the scatter is below 2^scatter_bits
-    int32_t spectral_seqs;     // sequences per block of the warp-form spectral passes; 0: the fixed shape
+    int32_t spectral_seqs;     // sequences per block of the spectral passes (sides 64..256); 0: the fixed shape
     // host-side permutations for test hooks
     int32_t *h_slot_of_pin;    // [P]
     int32_t *h_net_of_internal;// [E]
@@ -242,8 +242,8 @@ bool packed_place_launch(const PackedLaunch &l, const unsigned char *dev, cudaSt
 cudaError_t ctx_alloc(void **p, size_t bytes, cudaStream_t s);
 
 // spectral engine for the standalone solve
-// The sequences-per-block alternatives of the warp-form spectral passes (sides
-// 64..256) that a batch's autotuner times against the fixed shape (four).
+// The sequences-per-block alternatives of the spectral passes (sides
+// 64..256) that a batch's autotuner times against the fixed shape.
 constexpr int kSeqCandidates[2] = {2, 8};
 struct SpectralPlan {
     int32_t m, n, logm, logn;
@@ -254,7 +254,7 @@ struct SpectralPlan {
     double *partials;
     DevState *st;
     cudaStream_t stream;
-    // sequences per block of the warp-form passes (sides 64..256): 0 for the
+    // sequences per block of the passes (sides 64..256): 0 for the
     // fixed shape, else one a batch's autotuner chose (2 or 8)
     int32_t seqs = 0;
 };
@@ -280,7 +280,7 @@ struct SpectralArgs {
 int spectral_row_blocks(const SpectralPlan &p);   // how many those are
 int map_rho_blocks(size_t mn);                    // ... for launch_map_rho
 void launch_spectral_plan(const SpectralPlan &p, const SpectralArgs &a);
-// The warp-form passes (sides 64..256) of many solves as packed launches, one
+// The passes (sides 64..256) of many solves as packed launches, one
 // per template variant in use (k_spectral.cu): kind PK_ROWS_DCT_W, PK_COLS_W or
 // PK_ROWS_INV_W.
 struct SpectralJob {

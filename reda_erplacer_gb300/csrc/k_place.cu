@@ -245,8 +245,9 @@ __device__ __forceinline__ Df wa_exact(const WaArgs &a, int net_begin, int net_c
 }
 
 // All degree classes in one launch: blocks [cls_block[k], cls_block[k+1]) serve
-// class k.  The block partials of the HPWL total are summed in double-float by
-// the last block to finish (fixed order, src/hpwl.rs:341-342).
+// class k.  The block partials of the HPWL total are summed in double-float, in a
+// fixed order (src/hpwl.rs:341-342): by the last block to finish, or inside a whole
+// step by its tail (step_tail).
 struct WaClasses {
     int begin[kNumClasses], count[kNumClasses], general[kNumClasses], slot0[kNumClasses];
     int block0[kNumClasses + 1];
