@@ -17,6 +17,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <nvtx3/nvToolsExt.h>
 
 #include "erp_internal.cuh"
@@ -831,8 +833,6 @@ extern "C" erp_status erp_step(erp_ctx *ctx, erp_step_stats *stats) {
     return ERP_OK;
 }
 
-// The device address of a registered (pinned, device-mapped) host buffer, or
-// nullptr for any other memory.
 // p[0, n) as device-mapped host memory (registered or cudaHostAlloc'd), or
 // nullptr.  Both the first and the last element must be mapped, contiguously,
 // so a registration shorter than the array falls back to copies instead of the
@@ -849,6 +849,28 @@ static float *mapped_host(float *p, int n) {
     if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
     float *d = static_cast<float *>(a.devicePointer);
     return b.devicePointer == static_cast<void *>(d + (n - 1)) ? d : nullptr;
+}
+
+// As mapped_host, where the whole array lies in one allocation or registration: for
+// the entry points whose contract allows any host memory, two registrations with a gap
+// between them among it.  Others are copied.
+static float *mapped_whole(float *p, int n) {
+    static const auto query = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return reinterpret_cast<PFN_cuPointerGetAttribute_v4000>(fn);
+    }();
+    float *d = mapped_host(p, n);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(d);
+    if (!d || !query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        return nullptr;
+    return at >= start && at - start <= size && sizeof(float) * (size_t)n <= size - (at - start) ? d : nullptr;
 }
 
 extern "C" erp_status erp_step_host(erp_ctx *ctx, float *x, float *y, erp_step_stats *stats) {
@@ -965,7 +987,7 @@ extern "C" erp_status erp_set_scalars(erp_ctx *ctx, int32_t iteration, float gam
 extern "C" erp_status erp_get_positions(erp_ctx *ctx, float *x, float *y) {
     CTX_CHECK();
     if (!x || !y) return ERP_EINVAL;
-    float *dx = mapped_host(x, c.N), *dy = mapped_host(y, c.N);
+    float *dx = mapped_whole(x, c.N), *dy = mapped_whole(y, c.N);
     if (dx && dy) {
         launch_xy_to_host(c, dx, dy);
         CK(cudaGetLastError());
@@ -1286,7 +1308,7 @@ extern "C" erp_status erp_checkpoint(erp_ctx *ctx, void *buf, size_t bytes) {
 // they lie on float boundaries, else nullptr (the arrays are copied).
 static const float *mapped_checkpoint(const char *arrays, int n) {
     if ((reinterpret_cast<uintptr_t>(arrays) & 3) || n > INT_MAX / kCkptArrays) return nullptr;
-    return mapped_host(reinterpret_cast<float *>(const_cast<char *>(arrays)), n * kCkptArrays);
+    return mapped_whole(reinterpret_cast<float *>(const_cast<char *>(arrays)), n * kCkptArrays);
 }
 
 extern "C" erp_status erp_restore(erp_ctx *ctx, const void *buf, size_t bytes) {

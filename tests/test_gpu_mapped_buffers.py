@@ -51,3 +51,28 @@ def test_mapped_and_other_memory_agree(cells):
         for buf, o in ((x, ox), (y, oy)):
             assert (buf[:o] == -7.0).all() and (buf[o + n:] == -7.0).all()
     p.close()
+
+
+def test_registered_memory():
+    """Arrays inside a registration of the caller's."""
+    import torch
+    import reda_erplacer_gb300 as R
+    rt = torch.cuda.cudart()
+    p = R.Placement(small_synth(5000, seed=3, macros=1, io=20), (64, 64), 1.0, start_mode=1)
+    blob, n = np.frombuffer(p.checkpoint(), np.uint8), p.N
+    p.run(2)
+    want = [a.copy() for a in p.positions()]
+    raw = np.zeros(blob.nbytes + 16384, np.uint8)
+    raw = raw[(-raw.ctypes.data) % 4096:][:(blob.nbytes + 8192) // 4096 * 4096]
+    assert int(rt.cudaHostRegister(raw.ctypes.data, raw.nbytes, 0)) == 0
+    try:
+        src = raw[-blob.nbytes:]   # ends with the registration
+        src[:] = blob
+        assert p.lib.erp_restore(p.h, src.ctypes.data, src.nbytes) == 0
+        p.run(2)
+        x, y = raw[:4 * n].view(np.float32), raw[-4 * n:].view(np.float32)
+        assert p.lib.erp_get_positions(p.h, x.ctypes.data_as(F32P), y.ctypes.data_as(F32P)) == 0
+        assert np.array_equal(x, want[0]) and np.array_equal(y, want[1])
+    finally:
+        assert int(rt.cudaHostUnregister(raw.ctypes.data)) == 0
+    p.close()
