@@ -516,7 +516,6 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     ap.add(&c.partials, kMaxPartials);
     ap.add(&c.part_wl, kMaxPartials);
     ap.add(&c.part_ovf, kMaxRowBlocks);
-    c.max_partials = kMaxPartials;
     ap.add(&c.st, 1);
     ap.add(&c.tw_m, c.m);
     ap.add(&c.tw_n, c.n);

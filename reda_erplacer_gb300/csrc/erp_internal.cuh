@@ -137,7 +137,6 @@ struct Ctx {
     // --- reductions ---
     double *partials;          // kMaxPartials
     double *part_wl, *part_ovf;   // [kMaxPartials], [kMaxRowBlocks]: a step's HPWL and overflow block sums
-    int32_t max_partials;
     DevState *st;
     DevState *h_st;            // pinned host mirror
     void *arena;               // the one allocation that holds every device array above
