@@ -119,7 +119,7 @@ cudaError_t ctx_alloc(void **p, size_t bytes, cudaStream_t s) {
 
 namespace {
 
-bool pow2_ok(int v) { return v >= 16 && v <= 4096 && (v & (v - 1)) == 0; }
+bool pow2_ok(int v) { return v >= kGridMin && v <= kGridMax && (v & (v - 1)) == 0; }
 
 cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (!bytes) return cudaSuccess;
@@ -507,8 +507,8 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     ap.add(&c.sratio, NM);
     ap.add(&c.sort_key, NM);
     ap.add(&c.sort_rank, NM);
-    ap.add(&c.sort_hist, scatter_tiles(c.m, c.n));
-    ap.add(&c.sort_start, scatter_tiles(c.m, c.n));
+    ap.add(&c.sort_hist, sort_tiles(c.m, c.n));
+    ap.add(&c.sort_start, sort_tiles(c.m, c.n));
     ap.add(&c.dmap, mn);
     float **maps[] = {&c.initial, &c.rho, &c.t1, &c.tx, &c.ty, &c.tp, &c.psi};
     for (float **a : maps) ap.add(a, mn);
@@ -579,7 +579,7 @@ static erp_status create_impl(const erp_design *d, const erp_params *pp, Ctx &c)
     CK(cudaMemcpyAsync(c.st, c.h_st, sizeof(DevState), cudaMemcpyHostToDevice, c.stream));
     launch_pack_xy(c);
     CK(cudaMemsetAsync(c.n_items, 0, sizeof(int32_t), c.stream));   // without movable cells there are none
-    launch_scatter_order(c, c.stream);
+    CK(launch_scatter_order(c, c.stream));
     c.sort_age = 0;
     // fixed-cell initial density (src/epotential.rs:127-140)
     launch_initial_density(c, nullptr, nullptr, nullptr, nullptr);
@@ -799,18 +799,17 @@ static erp_status ensure_graph(Ctx &c) {
 
 // The scatter order follows the cells every kSortEvery steps (a stale order is
 // still correct, only slower).
-static void refresh_scatter_order(Ctx &c, int steps, cudaStream_t s) {
+static cudaError_t refresh_scatter_order(Ctx &c, int steps, cudaStream_t s) {
     c.sort_age += steps;
-    if (c.sort_age >= kSortEvery) {
-        launch_scatter_order(c, s);
-        c.sort_age = 0;
-    }
+    if (c.sort_age < kSortEvery) return cudaSuccess;
+    c.sort_age = 0;
+    return launch_scatter_order(c, s);
 }
 
 static erp_status enqueue_step(Ctx &c) {
     erp_status s = ensure_graph(c);
     if (s != ERP_OK) return s;
-    refresh_scatter_order(c, 1, c.stream);
+    CK(refresh_scatter_order(c, 1, c.stream));
     if (c.map_dirty) {
         CK(cudaMemsetAsync(c.dmap, 0, sizeof(unsigned long long) * (size_t)c.m * c.n, c.stream));
         c.map_dirty = false;
@@ -1854,11 +1853,14 @@ static erp_status batch_sort_graph(erp_batch *b, const std::vector<char> &active
             if (!active[i]) continue;
             Ctx &c = b->ctx[i]->c;
             cudaStreamWaitEvent(c.stream, fork, 0);
-            launch_scatter_order(c, c.stream);
+            const cudaError_t eo = launch_scatter_order(c, c.stream);
+            if (e == cudaSuccess) e = eo;
             cudaEventRecord(joins[i], c.stream);
             cudaStreamWaitEvent(b->master, joins[i], 0);
         }
-        e = cudaStreamEndCapture(b->master, &g);
+        const cudaError_t ec = cudaStreamEndCapture(b->master, &g);
+        if (ec == cudaSuccess && e != cudaSuccess) cudaGraphDestroy(g);
+        if (e == cudaSuccess) e = ec;
         if (e == cudaSuccess) {
             e = cudaGraphInstantiate(&b->sort_graph, g, 0);
             cudaGraphDestroy(g);
@@ -2044,7 +2046,7 @@ extern "C" erp_status erp_estimate_footprint(const erp_design *d, const erp_para
     b += al(4 * P) + 2 * al(8 * P) + al(4 * (E + 1)) + al(4 * E) + al(4 * (NM + 1)) + al(4 * movable_pins);
     b += al(8 * mn) + 7 * al(4 * mn) + al(8 * mn) + 2 * al(8 * (int64_t)kMaxPartials) +
          al(8 * (int64_t)kMaxRowBlocks) + al(sizeof(DevState));
-    b += 4 * al(4 * (int64_t)NM) + al(16 * (int64_t)scatter_items_max((int)NM, m, n)) + 512 + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)scatter_tiles(m, n));   // scatter order
+    b += 4 * al(4 * (int64_t)NM) + al(16 * (int64_t)scatter_items_max((int)NM, m, n)) + 512 + al(16 * (int64_t)NM) + 2 * al(4 * (int64_t)sort_tiles(m, n));   // scatter order
     b += al(4 * (NM + 4)) + al(8 * (NM + 4));   // its inverse, the density gradient in that order
     b += 2 * (al(8 * m) + al(8 * n)) + al(4 * m) + al(4 * n);
     if (pp && pp->precision != ERP_PREC_FP32) {   // tensor-core plan: 4 transforms per axis + 7 map buffers
@@ -2410,7 +2412,11 @@ static erp_status server_launch_round(erp_server *sv, int buf) {
             }
             j.form = 1;
         }
-        for (Ctx *c : xs) refresh_scatter_order(*c, sv->p.chunk, sv->pstream);
+        for (Ctx *c : xs)
+            if (refresh_scatter_order(*c, sv->p.chunk, sv->pstream) != cudaSuccess) {
+                sv->err = "scatter-order launch failed";
+                return ERP_ECUDA;
+            }
         erp_status s = server_pack_slot(sv, buf, xs, ids);
         if (s != ERP_OK) return s;
         for (int k = 0; k < sv->p.chunk; ++k)
@@ -2435,7 +2441,10 @@ static erp_status server_launch_round(erp_server *sv, int buf) {
             sv->err = c.err;
             return s;
         }
-        refresh_scatter_order(c, sv->p.chunk, c.stream);
+        if (refresh_scatter_order(c, sv->p.chunk, c.stream) != cudaSuccess) {
+            sv->err = "scatter-order launch failed";
+            return ERP_ECUDA;
+        }
         for (int k = 0; k < sv->p.chunk; ++k)
             if (cudaGraphLaunch(c.graph, c.stream) != cudaSuccess) {
                 sv->err = "job graph launch failed";

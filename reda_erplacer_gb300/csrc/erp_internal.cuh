@@ -12,6 +12,7 @@
 
 #include "erplacer.h"
 #include "packed.h"
+#include "sorttiles.h"
 
 namespace erp {
 
@@ -171,9 +172,8 @@ void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool 
 constexpr int kFieldPairCells = 131072;   // alone, designs of this many movable cells interleave (see k_force)
 void set_field_pairs(Ctx &c, bool pairs);
 int overflow_blocks(const Ctx &c);   // block sums the overflow has in this context's step
-void launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
+cudaError_t launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
 void launch_scatter_items(Ctx &c, cudaStream_t s);   // its work items again, after scatter_cells changed
-int scatter_tiles(int m, int n);
 int scatter_items_max(int NM, int m, int n);
 void launch_xy_from_host(Ctx &c, const float *hx, const float *hy);   // device-mapped host x, y -> x, y, xy
 void launch_restore(Ctx &c, const float *src, const DevState &state);   // a checkpoint's arrays in device-mapped host memory

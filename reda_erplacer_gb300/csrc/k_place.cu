@@ -423,7 +423,7 @@ __device__ __forceinline__ float tri_clamped(float x, float s, int k, float bs) 
 // contributions find the window.
 constexpr int kFollowCells = 131072;
 constexpr int kWin = 48;
-constexpr int kSortTile = 32, kSortPad = 8;
+constexpr int kSortPad = 8;
 static_assert(kSortTile + 2 * kSortPad == kWin, "the window covers a tile and its pads");
 constexpr int kTableLog = 8, kTable = 1 << kTableLog;   // out-of-window bin table (open, no probing)
 constexpr unsigned kEmpty = 0xffffffffu;                 // bin indices are < 4096 * 4096
@@ -808,8 +808,6 @@ __global__ void __launch_bounds__(kThreads) k_sort_place(int NM, const int32_t *
     }
 }
 
-int scatter_tiles(int m, int n) { return ((m + kSortTile - 1) / kSortTile) * ((n + kSortTile - 1) / kSortTile); }
-
 static cudaError_t packed_prepare();
 cudaError_t place_prepare() {
     cudaError_t e = cudaSuccess;
@@ -817,6 +815,8 @@ cudaError_t place_prepare() {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(scatter_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)density_scatter_smem(scatter_planes(v)));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_sort_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortCountSmem);
     if (e != cudaSuccess) return e;
     return packed_prepare();
 }
@@ -1640,8 +1640,8 @@ static int scatter_cap(const Ctx &c) {
 }
 
 // Items there can be: every tile with cells may hold one that is not full.
-static int scatter_items(const Ctx &c, int cap) { return std::min(scatter_tiles(c.m, c.n), c.NM) + (c.NM + cap - 1) / cap; }
-int scatter_items_max(int NM, int m, int n) { return std::min(scatter_tiles(m, n), NM) + (NM + 31) / 32; }
+static int scatter_items(const Ctx &c, int cap) { return std::min(sort_tiles(c.m, c.n), c.NM) + (c.NM + cap - 1) / cap; }
+int scatter_items_max(int NM, int m, int n) { return std::min(sort_tiles(m, n), NM) + (NM + 31) / 32; }
 
 static int scatter_params(Ctx &c, ScatterP &p, int &variant) {
     const int cap = scatter_cap(c);
@@ -1661,21 +1661,29 @@ void launch_density_scatter(Ctx &c) {
 // The items of the current order again, after scatter_cells changed.
 void launch_scatter_items(Ctx &c, cudaStream_t s) {
     if (c.NM <= 0) return;
-    k_sort_scan<<<1, 1024, 0, s>>>(scatter_tiles(c.m, c.n), (c.n + kSortTile - 1) / kSortTile, c.m, c.n, scatter_cap(c),
+    k_sort_scan<<<1, 1024, 0, s>>>(sort_tiles(c.m, c.n), (c.n + kSortTile - 1) / kSortTile, c.m, c.n, scatter_cap(c),
                                    c.sort_hist, c.sort_start, c.items, c.n_items);
 }
 
-void launch_scatter_order(Ctx &c, cudaStream_t s) {
-    if (c.NM <= 0) return;
+cudaError_t launch_scatter_order(Ctx &c, cudaStream_t s) {
+    if (c.NM <= 0) return cudaSuccess;
     const int nty = (c.n + kSortTile - 1) / kSortTile;
-    const int ntiles = scatter_tiles(c.m, c.n);
-    cudaMemsetAsync(c.sort_hist, 0, sizeof(int32_t) * ntiles, s);
-    k_sort_count<<<(c.NM + 4 * kThreads - 1) / (4 * kThreads), kThreads, sizeof(int32_t) * ntiles, s>>>(
-        c.NM, c.xy, c.offx, c.offy, c.inv_bw, c.inv_bh, c.m, c.n, nty, ntiles, c.sort_key, c.sort_rank,
-        c.sort_hist);
+    const int ntiles = sort_tiles(c.m, c.n);
+    cudaError_t e = cudaMemsetAsync(c.sort_hist, 0, sizeof(int32_t) * ntiles, s);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((c.NM + 4 * kThreads - 1) / (4 * kThreads));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sort_count_smem(c.m, c.n);
+    cfg.stream = s;
+    // the placing pass indexes with what this one writes: without it, it must not run
+    e = cudaLaunchKernelEx(&cfg, k_sort_count, c.NM, (const float2 *)c.xy, (const float *)c.offx, (const float *)c.offy,
+                           c.inv_bw, c.inv_bh, (int)c.m, (int)c.n, nty, ntiles, c.sort_key, c.sort_rank, c.sort_hist);
+    if (e != cudaSuccess) return e;
     launch_scatter_items(c, s);
     k_sort_place<<<grid_for(c.NM), kThreads, 0, s>>>(c.NM, c.sort_key, c.sort_rank, c.sort_start, c.offx, c.offy,
                                                      c.cw, c.ch, c.ratio, c.perm, c.pos, c.soff, c.sratio);
+    return cudaSuccess;
 }
 
 void launch_initial_density(Ctx &c, const float *, const float *, const float *, const float *) {
