@@ -384,7 +384,10 @@ erp_status erp_profile_stages(erp_ctx *ctx, int32_t reps, float *ms_out);
 /* ---- standalone spectral solve (the Poisson part of compute_potential,
  * src/epotential.rs:284-343) on device buffers, for the isolated-solve
  * workload.  All pointers are device pointers of m*n floats; potential may be
- * NULL. ---- */
+ * NULL.  Outputs may start on any boundary of floats (in the tensor-core
+ * precisions 32-byte boundaries are the fastest); rho_dev too, except for
+ * ERP_PREC_TF32_GEMM, whose bulk loads take it on a 16-byte boundary only
+ * (otherwise ERP_ECUDA, nothing launched). ---- */
 typedef struct erp_spectral erp_spectral;
 erp_status erp_spectral_create(int32_t m, int32_t n, float bin_w, float bin_h, int32_t precision,
                                void *stream, erp_spectral **out);

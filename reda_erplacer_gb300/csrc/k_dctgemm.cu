@@ -58,7 +58,7 @@ struct GemmEpi {
     int mode;                // 0: plain store, 1: weighted spectra (planes)
     int split;               // store bf16 hi/lo instead of fp32
     int lo_first;            // BF16x3: the product lo.hi before hi.lo
-    int wide;                // every output row starts on a 32-byte boundary
+    int unit;                // bytes per store: every output row starts on such a boundary (32, 16 or 4)
     int nplanes;             // weighted mode: planes x, y (, p)
     float alpha;             // scale applied before storing
     int ldc;                 // row stride of the stored matrix (elements)
@@ -142,16 +142,20 @@ __device__ __forceinline__ void store_sector(void *p, const uint32_t (&r)[8]) {
                  "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void store_words(uint32_t *p, const uint32_t (&r)[8], int wide) {
-    if (wide) {
+// eight words, `unit` bytes at a time (the same for a whole launch)
+__device__ __forceinline__ void store_words(uint32_t *p, const uint32_t (&r)[8], int unit) {
+    if (unit == 32) {
         store_sector(p, r);
-    } else {
+    } else if (unit == 16) {
         reinterpret_cast<uint4 *>(p)[0] = make_uint4(r[0], r[1], r[2], r[3]);
         reinterpret_cast<uint4 *>(p)[1] = make_uint4(r[4], r[5], r[6], r[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) p[k] = r[k];
     }
 }
 // 32 consecutive elements of a matrix from element `at` on: fp32, or bf16 hi and lo
-__device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, const float (&x)[32], int split, int wide) {
+__device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, const float (&x)[32], int split, int unit) {
     if (!split) {
         uint32_t *o = static_cast<uint32_t *>(out[0]) + at;
 #pragma unroll
@@ -159,7 +163,7 @@ __device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, cons
             uint32_t r[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) r[k] = __float_as_uint(x[8 * q + k]);
-            store_words(o + 8 * q, r, wide);
+            store_words(o + 8 * q, r, unit);
         }
         return;
     }
@@ -175,8 +179,8 @@ __device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, cons
             memcpy(&h[k], &hi, 4);
             memcpy(&l[k], &lo, 4);
         }
-        store_words(oh + 8 * q, h, wide);
-        store_words(ol + 8 * q, l, wide);
+        store_words(oh + 8 * q, h, unit);
+        store_words(ol + 8 * q, l, unit);
     }
 }
 
@@ -314,8 +318,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_nt(const __grid_consta
     } else if (warp >= 2) {
         // Epilogue: warps w and w + 4 share the TMEM lanes of quarter w mod 4 and take
         // alternate blocks of 32 columns.  Each thread holds 32 columns of its row at a
-        // time and stores them itself, a 32-byte sector per instruction (16 bytes where
-        // a caller's buffer allows no more): no staging, and the weights of a row share
+        // time and stores them itself, a 32-byte sector per instruction (16 or 4 bytes
+        // where a caller's buffer allows no more): no staging, and the weights of a row share
         // its wu.  The next tile's products run meanwhile in the other accumulator.
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const float al = epi.alpha;
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_nt(const __grid_consta
                 for (int j = 0; j < 32; ++j) v[j] *= al;
                 const size_t at = (size_t)gr * epi.ldc + tl.n + c0;
                 if (epi.mode == 0) {
-                    store_row(epi.out[tl.z], at, v, epi.split, epi.wide);
+                    store_row(epi.out[tl.z], at, v, epi.split, epi.unit);
                     continue;
                 }
                 // weighted spectra: row u = gr, column gc (planes x, y, p)
@@ -360,9 +364,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_nt(const __grid_consta
                         v[j] = x * ik;
                     }
                 }
-                store_row(epi.out[0], at, px, epi.split, epi.wide);
-                store_row(epi.out[1], at, py, epi.split, epi.wide);
-                if (epi.nplanes > 2) store_row(epi.out[2], at, v, epi.split, epi.wide);
+                store_row(epi.out[0], at, px, epi.split, epi.unit);
+                store_row(epi.out[1], at, py, epi.split, epi.unit);
+                if (epi.nplanes > 2) store_row(epi.out[2], at, v, epi.split, epi.unit);
             }
             tc_fence_before();
             __syncwarp();
@@ -658,7 +662,7 @@ cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy
     ep.status = status ? status : P.h_status;
     ep.status_on_host = status ? 0 : 1;
     ep.split = split ? 1 : 0;
-    ep.wide = 1;   // the plan's own buffers
+    ep.unit = 32;   // the plan's own buffers
     // G1: Z^T = C_n rho^T [n][m] (the operands' order gives the transpose; lo_first keeps
     // the order of the products rho hi . C_n lo, rho lo . C_n hi)
     ep.mode = 0; ep.lo_first = 1; ep.alpha = 1.0f; ep.ldc = m;
@@ -676,11 +680,13 @@ cudaError_t dctgemm_solve(DctGemmPlan &P, const float *rho, float *fx, float *fy
     // G4: field_x = S_m Z_x, field_y = D_m Z_y, psi = D_m Z_p, fp32 [m][n], the caller's buffers
     ep.split = 0; ep.lo_first = 0; ep.ldc = n;
     float *outs[3] = {fx, fy, psi};
+    uintptr_t low = 0;
     for (int k = 0; k < nk; ++k) {
         ep.out[k][0] = outs[k];
         ep.out[k][1] = nullptr;
-        if (reinterpret_cast<uintptr_t>(outs[k]) & 31) ep.wide = 0;
+        low |= reinterpret_cast<uintptr_t>(outs[k]);
     }
+    ep.unit = low & 15 ? 4 : (low & 31 ? 16 : 32);
     if ((e = run_gemm(P, P.g4[nk - 2], ep, m, n, m, nk, P.bn4[nk - 2], s)) != cudaSuccess) return e;
     return cudaSuccess;
 }

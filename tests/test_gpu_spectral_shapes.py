@@ -87,3 +87,32 @@ def test_contraction_tiles(m, n, precision):
     for r in results[1:]:
         for a, b in zip(results[0], r):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("m,n", [(128, 128), (256, 512), (1024, 2048)])
+def test_contraction_outputs_on_4_byte_boundaries(m, n, precision):
+    """The tensor-core solve into buffers that start on any boundary of floats, each
+    its own: the bits of aligned ones, nothing written outside, the density where it
+    is (BF16x3 takes it on 4-byte boundaries too)."""
+    import torch
+    import reda_erplacer_gb300 as R
+    rng = np.random.default_rng(m + 3 * n)
+    rho = torch.from_numpy((0.7 + 0.3 * rng.random(m * n)).astype(np.float32))
+    s = R.SpectralSolver(m, n, 1.3, 1.0, stream=torch.cuda.current_stream().cuda_stream, precision=precision)
+    want = None
+    for offsets in ((0, 0, 0), (1, 0, 0), (0, 2, 3), (3, 1, 2), (2, 2, 2)):
+        buf = [torch.full((m * n + 8,), -7.0, dtype=torch.float32, device="cuda") for _ in range(3)]
+        at = [b[o:o + m * n] for b, o in zip(buf, offsets)]
+        src = torch.zeros(m * n + 8, dtype=torch.float32, device="cuda")
+        skip = offsets[0] if precision == 2 else 0
+        src[skip:skip + m * n] = rho.cuda()
+        s.solve(src[skip:].data_ptr(), *[t.data_ptr() for t in at])
+        torch.cuda.synchronize()
+        got = [t.clone() for t in at]
+        want = want or got
+        for a, b in zip(want, got):
+            assert torch.equal(a, b)
+        for b, o in zip(buf, offsets):
+            assert bool((b[:o] == -7.0).all()) and bool((b[o + m * n:] == -7.0).all())
+    s.close()
