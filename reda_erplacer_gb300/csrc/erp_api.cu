@@ -831,14 +831,14 @@ extern "C" erp_status erp_step(erp_ctx *ctx, erp_step_stats *stats) {
     return ERP_OK;
 }
 
-// p[0, n) as device-mapped host memory (registered or cudaHostAlloc'd), or
-// nullptr.  Both the first and the last element must be mapped, contiguously,
+// p[0, n) as device-mapped host memory (registered or cudaHostAlloc'd) on a boundary
+// of floats, which a kernel's accesses need and a copy does not, or nullptr.  Both the first and the last element must be mapped, contiguously,
 // so a registration shorter than the array falls back to copies instead of the
 // device running past it.  (A range that starts and ends in two different
 // registrations with unregistered memory between them is not detected: the
 // caller's contract is one registration per array.)
 static float *mapped_host(float *p, int n) {
-    if (n <= 0) return nullptr;
+    if (n <= 0 || reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
     cudaPointerAttributes a, b;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + (n - 1)) != cudaSuccess) {
         cudaGetLastError();
@@ -1305,7 +1305,7 @@ extern "C" erp_status erp_checkpoint(erp_ctx *ctx, void *buf, size_t bytes) {
 // The device address of a checkpoint's arrays where the buffer is device-mapped and
 // they lie on float boundaries, else nullptr (the arrays are copied).
 static const float *mapped_checkpoint(const char *arrays, int n) {
-    if ((reinterpret_cast<uintptr_t>(arrays) & 3) || n > INT_MAX / kCkptArrays) return nullptr;
+    if (n > INT_MAX / kCkptArrays) return nullptr;
     return mapped_whole(reinterpret_cast<float *>(const_cast<char *>(arrays)), n * kCkptArrays);
 }
 

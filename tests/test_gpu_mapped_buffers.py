@@ -76,3 +76,34 @@ def test_registered_memory():
     finally:
         assert int(rt.cudaHostUnregister(raw.ctypes.data)) == 0
     p.close()
+
+
+@pytest.mark.parametrize("cells", [901, 900])
+def test_positions_off_the_boundary_of_floats(cells):
+    """Pinned arrays that start between two floats (a record's field, say) are copied:
+    no kernel may store there.  Reading the positions, and a host-owned step."""
+    import reda_erplacer_gb300 as R
+    p = R.Placement(small_synth(cells, seed=9, macros=2, io=30), (64, 64), 1.0, start_mode=1)
+    p.run(3)
+    want = [a.copy() for a in p.positions()]
+    n = p.N
+
+    def at(shift):
+        raw = pinned(4 * n + 16)
+        raw[:] = 0xEE
+        return raw, C.cast(raw.ctypes.data + shift, F32P), raw[shift:shift + 4 * n]
+
+    for sx, sy in ((1, 0), (0, 2), (3, 1), (2, 2)):
+        (rx, px, vx), (ry, py, vy) = at(sx), at(sy)
+        assert p.lib.erp_get_positions(p.h, px, py) == 0
+        assert vx.tobytes() == want[0].tobytes() and vy.tobytes() == want[1].tobytes()
+        for raw, s in ((rx, sx), (ry, sy)):
+            assert (raw[:s] == 0xEE).all() and (raw[s + 4 * n:] == 0xEE).all()
+    blob = p.checkpoint()
+    p.step()
+    want = [a.copy() for a in p.positions()]
+    p.restore(blob)
+    assert p.lib.erp_get_positions(p.h, px, py) == 0
+    assert p.lib.erp_step_host(p.h, px, py, None) == 0
+    assert vx.tobytes() == want[0].tobytes() and vy.tobytes() == want[1].tobytes()
+    p.close()
