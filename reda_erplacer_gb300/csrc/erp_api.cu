@@ -986,7 +986,10 @@ extern "C" erp_status erp_get_positions(erp_ctx *ctx, float *x, float *y) {
     CTX_CHECK();
     if (!x || !y) return ERP_EINVAL;
     float *dx = mapped_whole(x, c.N), *dy = mapped_whole(y, c.N);
-    if (dx && dy) {
+    // arrays that share memory keep the order of two copies: y is written last
+    const uintptr_t ax = reinterpret_cast<uintptr_t>(x), ay = reinterpret_cast<uintptr_t>(y);
+    const bool apart = (ax > ay ? ax - ay : ay - ax) >= sizeof(float) * (uintptr_t)c.N;
+    if (dx && dy && apart) {
         launch_xy_to_host(c, dx, dy);
         CK(cudaGetLastError());
     } else {

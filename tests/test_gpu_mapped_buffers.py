@@ -107,3 +107,20 @@ def test_positions_off_the_boundary_of_floats(cells):
     assert p.lib.erp_step_host(p.h, px, py, None) == 0
     assert vx.tobytes() == want[0].tobytes() and vy.tobytes() == want[1].tobytes()
     p.close()
+
+
+@pytest.mark.parametrize("shift", [0, 1, 4, 100])
+def test_positions_into_arrays_that_share_memory(shift):
+    """A caller that wants one coordinate may give one array for both, or two that
+    overlap: y is written after x, in pinned memory as in any other."""
+    import reda_erplacer_gb300 as R
+    p = R.Placement(small_synth(20001, seed=9, macros=2, io=30), (64, 64), 1.0, start_mode=1)
+    p.run(3)
+    want, n = [a.copy() for a in p.positions()], p.N
+    for buf in (np.zeros(n + shift, np.float32), pinned(4 * (n + shift)).view(np.float32)):
+        for x, y in ((buf[:n], buf[shift:]), (buf[shift:], buf[:n])):
+            assert p.lib.erp_get_positions(p.h, x.ctypes.data_as(F32P), y.ctypes.data_as(F32P)) == 0
+            expect = np.concatenate([want[0][:shift], want[1]]) if y is not x and y.ctypes.data >= x.ctypes.data \
+                else np.concatenate([want[1], want[0][n - shift:]])
+            assert np.array_equal(buf, expect)
+    p.close()
