@@ -1055,14 +1055,10 @@ extern "C" erp_status erp_get_array(erp_ctx *ctx, erp_array which, void *dst, si
     case ERP_ARR_FIELD_Y:
         src = which == ERP_ARR_FIELD_X ? c.fx : c.fy;
         need = sizeof(float) * mn;
-        if (c.field_pairs) {   // interleaved on the device
-            if (bytes < need) { c.err = "destination too small"; return ERP_EINVAL; }
-            std::vector<float2> f(mn);
-            CK(cudaMemcpyAsync(f.data(), c.fx, sizeof(float2) * mn, cudaMemcpyDeviceToHost, c.stream));
-            CK(cudaStreamSynchronize(c.stream));
-            float *o = (float *)dst;
-            for (size_t k = 0; k < mn; ++k) o[k] = which == ERP_ARR_FIELD_X ? f[k].x : f[k].y;
-            return ERP_OK;
+        if (c.field_pairs && bytes >= need) {   // interleaved: a map of its own, in the solve's scratch
+            launch_field_map(c, which == ERP_ARR_FIELD_X ? 0 : 1, c.t1);
+            CK(cudaGetLastError());
+            src = c.t1;
         }
         break;
     case ERP_ARR_POTENTIAL: src = c.psi; need = sizeof(float) * mn; break;

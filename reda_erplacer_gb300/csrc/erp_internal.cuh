@@ -171,6 +171,7 @@ void launch_spectral(Ctx &c, bool zero_map, bool store_rho, bool want_psi, bool 
 // a stage uses them): interleaved, or (always with the tensor-core solve) two maps.
 constexpr int kFieldPairCells = 131072;   // alone, designs of this many movable cells interleave (see k_force)
 void set_field_pairs(Ctx &c, bool pairs);
+void launch_field_map(Ctx &c, int which, float *out);   // interleaved fields: field_x (0) or field_y (1) as a map
 int overflow_blocks(const Ctx &c);   // block sums the overflow has in this context's step
 cudaError_t launch_scatter_order(Ctx &c, cudaStream_t s);   // recompute the scatter order from the current positions
 void launch_scatter_items(Ctx &c, cudaStream_t s);   // its work items again, after scatter_cells changed

@@ -51,3 +51,39 @@ def test_fields_and_force_at_the_size_rule(cells):
     finally:
         g.close()
         o.close()
+
+
+def test_interleaved_fields_read_back():
+    """The fields of an interleaved context, as maps: the bits of the same design's two
+    maps, into ordinary and page-locked arrays, x and y in either order; a short
+    destination is refused; the solve's scratch that the maps pass through is free for
+    the next step."""
+    import ctypes as C
+    import torch
+    import reda_erplacer_gb300 as R
+    bins = [(64, 64), (64, 128), (256, 64), (128, 128)]
+    designs = [small_synth(800 + 300 * i, seed=70 + i, macros=1) for i in range(4)]
+    b = R.Batch(designs, bins, 1.0, start_mode=1)
+    assert b.packed_instances() == 4
+    for steps in (5, 4):
+        b.run(steps)
+    for i, (d, (m, n)) in enumerate(zip(designs, bins)):
+        p = R.Placement(d, (m, n), 1.0, start_mode=1)
+        p.run(9)
+        ctx = C.c_void_p(b.lib.erp_batch_context(b.h, i))
+        pinned = torch.empty(m * n, pin_memory=True).numpy()
+        for name in ("FIELD_Y", "FIELD_X", "FIELD_Y"):
+            want = p.array(name)
+            for out in (np.zeros(m * n, np.float32), pinned):
+                out[:] = -7.0
+                to = out.ctypes.data_as(C.c_void_p)
+                assert b.lib.erp_get_array(ctx, R.lib.ARR[name], to, out.nbytes - 4) == R.lib.EINVAL
+                assert (out == -7.0).all()
+                assert b.lib.erp_get_array(ctx, R.lib.ARR[name], to, out.nbytes) == 0
+                assert np.abs(want).max() > 0 and np.array_equal(out, want)
+            b.lib.erp_step(ctx, None)
+            p.step()
+        for u, v in zip(b.positions(i), p.positions()):
+            assert np.array_equal(u, v)
+        p.close()
+    b.close()
