@@ -172,6 +172,17 @@ struct PairFft {
         if constexpr (kEarly) return ld_now(p);
         else return __ldg(p);
     }
+    // An element that the same kernel writes later (WRITTEN), or that no pass of it does.
+    template <bool WRITTEN>
+    static __device__ __forceinline__ float load_elem(const float *p) {
+        if constexpr (WRITTEN) {
+            float v;
+            asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+            return v;
+        } else {
+            return load(p);
+        }
+    }
     // A pair of the pass before: WRITTEN in the same kernel, or by an earlier one.
     template <bool WRITTEN>
     static __device__ __forceinline__ float2 load_pair(const float2 *p) {

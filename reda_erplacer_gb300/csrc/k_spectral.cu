@@ -387,7 +387,10 @@ struct RowsFwdP {
     double movable_area;
     int step;   // 1: inside a whole step, the overflow's block sums are left for its tail (k_nesterov_update)
 };
-template <int N, int P>
+// INNER (all three passes below): the whole solve is one kernel.  What a pass reads was
+// written earlier in it, or (the density, where a caller's output takes its place) is
+// written later, which rules the read-only path out.
+template <int N, int P, bool INNER = false>
 __device__ __forceinline__ void rows_fwd_body(const RowsFwdP &a, int bid, int nblk) {
     using F = PairFft<N, P>;
     DevState *__restrict__ st = a.st;
@@ -452,7 +455,7 @@ __device__ __forceinline__ void rows_fwd_body(const RowsFwdP &a, int bid, int nb
 #pragma unroll
         for (int j = 0; j < F::R1; ++j) {
             const int i = makhoul_elem(t + j * F::M, N);
-            v[j] = make_float2(F::load(a.rho_in + ra + i), F::load(a.rho_in + rb + i));
+            v[j] = make_float2(F::template load_elem<INNER>(a.rho_in + ra + i), F::template load_elem<INNER>(a.rho_in + rb + i));
         }
         F::load_tw1(w1, a.tw_n, t);
     }
@@ -507,8 +510,6 @@ struct ColsP {
     float scale4;
     const DevState * st;
 };
-// INNER (both passes below): their input was written earlier in the same kernel, which
-// rules the read-only path out.
 template <int N, int P, bool INNER = false>
 __device__ __forceinline__ void cols_body(const ColsP &a, int bid, int nblk) {
     using F = PairFft<N, P>;
@@ -704,7 +705,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(PairFft<N, 
     static_assert(PairFft<N, P>::THREADS == PairFft<M, P>::THREADS, "one block shape for all passes");
     static_assert(ROWS <= kSmallCtas && COLS <= kSmallCtas, "at most one block per CTA");
     const int cta = blockIdx.x;
-    if (cta < ROWS) rows_fwd_body<N, P>(p.fwd, cta, ROWS);
+    if (cta < ROWS) rows_fwd_body<N, P, true>(p.fwd, cta, ROWS);
     cluster_barrier();
     if (cta < COLS) cols_body<M, P, true>(p.cols, cta, COLS);
     cluster_barrier();

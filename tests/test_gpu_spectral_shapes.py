@@ -116,3 +116,25 @@ def test_contraction_outputs_on_4_byte_boundaries(m, n, precision):
         for b, o in zip(buf, offsets):
             assert bool((b[:o] == -7.0).all()) and bool((b[o + m * n:] == -7.0).all())
     s.close()
+
+
+@pytest.mark.parametrize("precision,m,n", [(0, 64, 64), (0, 64, 128), (0, 128, 64), (0, 128, 128), (0, 16, 64),
+                                           (0, 512, 256), (0, 4096, 64), (1, 256, 128), (2, 256, 128)])
+def test_output_in_the_densitys_place(precision, m, n):
+    """An output that overwrites the density (the density is read before any output is
+    written, in one launch or several): the bits of outputs of their own."""
+    import torch
+    import reda_erplacer_gb300 as R
+    rng = np.random.default_rng(m * 7 + n)
+    rho = torch.from_numpy((0.7 + 0.3 * rng.random(m * n)).astype(np.float32)).cuda()
+    s = R.SpectralSolver(m, n, 1.3, 1.0, stream=torch.cuda.current_stream().cuda_stream, precision=precision)
+    want = [torch.empty_like(rho) for _ in range(3)]
+    s.solve(rho.data_ptr(), *[t.data_ptr() for t in want])
+    for which in range(3):
+        out = [torch.empty_like(rho) for _ in range(3)]
+        out[which].copy_(rho)
+        s.solve(out[which].data_ptr(), *[t.data_ptr() for t in out])
+        torch.cuda.synchronize()
+        for a, b in zip(want, out):
+            assert torch.equal(a, b)
+    s.close()
