@@ -66,18 +66,33 @@ ERP_FXP_FN uint64_t fxp_rint_u64(float v) {
     return q;
 }
 
-// floor(x 2^-b) for x in [0, 2^(b + 23)) as a float and as an integer, by adding 2^23
-// rounded down; x - floor 2^b exactly.
-ERP_FXP_FN float fxp_high_part(float x, float inv_pow, float pow, uint32_t &high) {
+// a b + 2^23 rounded towards minus infinity, for a b in [0, 2^23).  On the host the sum
+// is formed in FP64, where nothing of it is lost that could reach the next integer (a is
+// a float, b a power of two), and rounded to the float below.
+ERP_FXP_FN float fxp_fma_down_2p23(float a, float b) {
 #if defined(__CUDA_ARCH__)
-    const float t = __fmaf_rd(x, inv_pow, 8388608.0f);
-    high = __float_as_uint(t) - 0x4b000000u;
-    return __fmaf_rn(-__fadd_rn(t, -8388608.0f), pow, x);
+    return __fmaf_rd(a, b, 8388608.0f);
 #else
-    const float f = __builtin_floorf(x * inv_pow);   // the product only moves the exponent
-    high = (uint32_t)f;
-    return (float)((double)x - (double)f * (double)pow);
+    const double sum = (double)a * (double)b + 8388608.0;
+    const float t = (float)sum;
+    return (double)t > sum ? fxp_bits_float(fxp_float_bits(t) - 1u) : t;
 #endif
+}
+ERP_FXP_FN float fxp_fma(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+    return __fmaf_rn(a, b, c);
+#else
+    return __builtin_fmaf(a, b, c);
+#endif
+}
+
+// floor(x 2^-b) for x in [0, 2^(b + 23)) as an integer, by adding 2^23 rounded down (the
+// sum's low bits are that integer); x - floor 2^b exactly.  The host runs the same
+// operations, so its test of the pieces is one of the device's arithmetic.
+ERP_FXP_FN float fxp_high_part(float x, float inv_pow, float pow, uint32_t &high) {
+    const float t = fxp_fma_down_2p23(x, inv_pow);
+    high = fxp_float_bits(t) - 0x4b000000u;
+    return fxp_fma(-(t - 8388608.0f), pow, x);
 }
 
 // rint(x) (round half to even, as fxp_rint_u64) as s0 + s1 2^B with s0 < 2^B, for x in
