@@ -138,3 +138,27 @@ def test_output_in_the_densitys_place(precision, m, n):
         for a, b in zip(want, out):
             assert torch.equal(a, b)
     s.close()
+
+
+@pytest.mark.parametrize("m,n", [(4096, 64), (64, 4096), (4096, 16), (4096, 2048), (2048, 4096)])
+def test_side_4096_against_64_bits(m, n):
+    """The longest transforms against the solve in 64 bits.  The bar is twice the error
+    that the oracle's own FP32 solve has on the same density: both round every product
+    and sum of transforms of the same lengths once, in other orders.  (An absolute bar
+    does not serve: of a density of white noise around 0.85 the rounding of the mean is
+    most of the error, and it grows with the grid.)"""
+    import torch
+    import reda_erplacer_gb300 as R
+    from oracle import erp_oracle as O
+    rng = np.random.default_rng(m * 3 + n)
+    rho = torch.from_numpy((0.7 + 0.3 * rng.random((m, n))).astype(np.float32))
+    want = O.poisson(rho.numpy().astype(np.float64), 1.3, 1.1, dtype=np.float64)
+    fp32 = O.poisson(rho.numpy(), 1.3, 1.1, dtype=np.float32)
+    s = R.SpectralSolver(m, n, 1.3, 1.1, stream=torch.cuda.current_stream().cuda_stream)
+    src, out = rho.cuda(), [torch.empty(m, n, dtype=torch.float32, device="cuda") for _ in range(3)]
+    s.solve(src.data_ptr(), *[t.data_ptr() for t in out])
+    torch.cuda.synchronize()
+    s.close()
+    flat = [[np.asarray(t, np.float64).ravel() for t in three] for three in ([t.cpu().numpy() for t in out], fp32, want)]
+    for got, theirs, ref in zip(*flat):
+        assert np.linalg.norm(got - ref) <= 2 * np.linalg.norm(theirs - ref)
