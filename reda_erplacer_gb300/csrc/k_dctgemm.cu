@@ -17,7 +17,8 @@
 // A launch whose result is wanted transposed (the K-major operand of the next one)
 // exchanges its operands instead: (A B^T)^T = B A^T, so every result is stored by rows.
 //
-// GEMM kernel: persistent CTAs, one per SM, over 128 x BN output tiles (tile_width).
+// GEMM kernel: persistent CTAs, one per SM (their registers allow no second), over
+// 128 x BN output tiles (tile_width).
 // Thread 0 issues TMA tile loads (128-byte swizzle) into a ring of shared-memory
 // stages; thread 32 issues the tcgen05.mma instructions into one of two FP32
 // accumulators of BN columns in tensor memory and releases each stage with
@@ -47,7 +48,7 @@ namespace erp {
 
 namespace {
 
-constexpr int kTile = 128;   // M and N of an output tile (TMEM lanes x columns)
+constexpr int kTile = 128;   // rows of an output tile (TMEM lanes); its columns are BN
 
 struct GemmMaps {            // per z: A (hi, lo) and B (hi, lo); lo only for BF16x3
     CUtensorMap a[3][2];
@@ -185,10 +186,12 @@ __device__ __forceinline__ void store_row(void *const (&out)[2], size_t at, cons
 }
 
 // Stage ring: A tile 128 x 128 bytes, B tile BN x 128 bytes (+ the lo parts
-// for BF16x3), as many stages as fit in 200 KB: one CTA per SM, which may then use
-// all of the SM's tensor memory.  TF32 up to 128 columns: 100 KB, two CTAs per SM with
-// 2 BN columns of tensor memory each (more stages measured no faster, and launches of
-// short grids start later with 200 KB: 1024 x 512 solve 52.6 against 50.3 us).
+// for BF16x3), as many stages as fit in 200 KB; TF32 up to 128 columns in 100 KB (more
+// stages measured no faster, and launches of short grids start later with 200 KB:
+// 1024 x 512 solve 52.6 against 50.3 us).  Tensor memory: 2 BN of the SM's 512 columns
+// per CTA.  Its registers (320 threads of 148) leave an SM room for one CTA; by shared
+// memory alone it would be two of the 100 KB form, and kMostPerSm times 2 BN columns fit
+// even then, so that no allocation waits for another's.
 template <int KIND, int BN>
 struct GemmCfg {
     static constexpr int kABytes = kTile * 128, kBBytes = BN * 128;
@@ -197,6 +200,8 @@ struct GemmCfg {
     static constexpr int kStages = kBudget * 1024 / kStageBytes;
     static constexpr int kBK = KIND == 0 ? 32 : 64;             // K elements per stage (128 bytes)
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
+    static constexpr int kMostPerSm = (int)(227 * 1024 / kSmem);
+    static_assert(kMostPerSm >= 1 && kMostPerSm * 2 * BN <= 512, "the accumulators of an SM's CTAs fit its tensor memory");
 };
 constexpr int kGemmThreads = 320;   // TMA warp, MMA warp, eight epilogue warps
 
@@ -255,7 +260,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_nt(const __grid_consta
         const Tile first = tile_at(blockIdx.x);
         for (int kt = 0; kt < ahead; ++kt) load_stage(first, kt, kt);
     }
-    if (warp == 1) {   // two accumulators of BN columns; one CTA per SM, so all 512 columns may be taken
+    if (warp == 1) {   // two accumulators of BN columns (GemmCfg: they fit)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base)),
                      "r"(2 * BN)
                      : "memory");
@@ -583,9 +588,9 @@ DctGemmPlan *dctgemm_create(int m, int n, float bin_w, float bin_h, int kind, cu
     if (ok) *P->h_status = 0;
     ok = ok && cudaMemcpy(P->wu, hu.data(), sizeof(float) * m, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(P->wv, hv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) == cudaSuccess;
-    // maps: G1 A = rho (per call for TF32, rho2 for BF16x3), B = C_n;  G2 A = C_m, B = Zt;
-    // G3 A = Aw[k], B = D_n / S_n / D_n;  G4 A = S_m / D_m / D_m, B = Zkt[k]
-    // G1 and G2 (one contraction per launch) use 128 x 64 tiles: twice the CTAs
+    // maps: G1 A = C_n, B = rho (per call for TF32, rho2 for BF16x3);  G2 A = C_m, B = Zt;
+    // G3 A = D_n / S_n / D_n, B = Aw[k];  G4 A = S_m / D_m / D_m, B = Zkt[k].  G1 and G3
+    // give their results transposed.
     P->bn[0] = tile_width(n, m, 1);
     P->bn[1] = tile_width(m, n, 1);
     ok = ok && set_maps(*P, P->g1.a[0], P->Cn, n, n) && set_maps(*P, P->g2.a[0], P->Cm, m, m) &&
