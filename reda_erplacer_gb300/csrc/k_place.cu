@@ -415,7 +415,12 @@ __device__ __forceinline__ float tri_clamped(float x, float s, int k, float bs) 
 // over 1024^2 bins, fresh order 41 -> 23 us (per-lane bin loops, 64-bin windows and
 // unaligned blocks before), all cells 20 bins further 41 -> 24 us (39 with the window
 // on the tile); crowded start 31.5 -> 27.7 us.  At 20,000 cells the mean's dependent
-// loads cost 0.5 of 6.6 us.  Tiles of 32 bins (48 before) also bring k_force from
+// loads cost 0.5 of 6.6 us.  Around the bound neither is faster throughout (us per step,
+// window on the tile / on the mean, cells crowded, half spread, spread): 60,000 cells
+// 40.0 / 38.8, 40.2 / 40.4, 40.2 / 43.7; 120,000 46.6 / 46.5, 46.0 / 45.9, 46.1 / 46.7;
+// 131,072 48.5 / 49.0, 49.5 / 49.2, 49.9 / 49.7; 200,000 55.4 / 57.0, 56.4 / 57.5,
+// 55.4 / 57.4; 300,000 65.9 / 64.2, 69.2 / 68.7, 66.3 / 68.7; 500,000 94.4 / 94.9,
+// 104.0 / 100.6, 103.1 / 103.8; the bound keeps the mean where cells move fast.  Tiles of 32 bins (48 before) also bring k_force from
 // 21 to 17 us at 1M cells.  Positions come from
 // the packed xy array; the stretched offsets, sizes and ratios were gathered
 // into the scatter order when it was computed (they never change).  Any
@@ -878,7 +883,11 @@ __device__ __forceinline__ float tri_raw(float x, float s, int k, float bs) {
 // 1024^2 bins: 17.2 -> 14.7 us with a fresh order, 28 -> 19 us in steps that move the
 // cells by tens of bins, against 1.4 us more in the solve's last pass; 550,000 cells in
 // 32 packed instances 17.3 -> 14.3 us.  One small design has too few warps for that to
-// matter and keeps two maps (20,000 cells: 4.4 against 5.2 us).
+// matter and keeps two maps (20,000 cells over 256^2 bins: 4.4 against 5.2 us).  Around
+// the bound, us per step with two maps / interleaved, cells crowded, half spread, spread:
+// 60,000 cells 40.4 / 38.2, 40.3 / 41.0, 40.2 / 41.7; 90,000 42.1 / 43.3, 41.9 / 42.7,
+// 42.3 / 43.9; 120,000 46.6 / 46.7, 47.0 / 45.4, 48.1 / 46.2; 131,072 51.3 / 48.7,
+// 50.6 / 50.4, 52.2 / 49.7; 200,000 59.3 / 57.0, 60.4 / 58.9, 59.3 / 57.2.
 struct ForceP {
     int NM;
     const int32_t * perm;
@@ -1554,7 +1563,9 @@ static int grid_for(int work, int cap = 152 * 8) {
     return g < 1 ? 1 : (g > cap ? cap : g);
 }
 
-constexpr int kWaBlocks = 152 * 4;   // k_wa's blocks that are resident at once
+// k_wa's blocks that are resident at once when it runs alone: its launch bounds' four on
+// each of the 152 SMs (in a step the density's branch takes some of that room).
+constexpr int kWaBlocks = 152 * 4;
 static_assert(kWaBlocks <= kMaxPartials, "a block sum per block");
 static int wa_params(Ctx &c, float gamma_arg, bool step, WaP &p) {
     WaArgs a;

@@ -358,7 +358,13 @@ __device__ __forceinline__ float2 dct2_pair(float2 z1, float2 z2, float2 e) {
 // e_{N-u} of e_u = (cos, -sin): the angle's complement to pi / 2
 __device__ __forceinline__ float2 ek_mirror(float2 e) { return make_float2(-e.y, -e.x); }
 
-// z[u] of the inverse from (X_a, X_b)[u] and (X_a, X_b)[N-u] (zero at u = 0)
+// z[u] of the inverse from (X_a, X_b)[u] and (X_a, X_b)[N-u] (zero at u = 0).  The
+// products with P are the rounded ones, those with Q go into the fused operation.  Other
+// orders are as accurate (eight were tried), but a placement's loop grows a difference of
+// one rounding: they spread the 20,000-cell run's HPWL at its least overflow over 2.3651e6
+// to 2.3767e6, about the two oracle forms' own 2.3698e6 and 2.3812e6, and the end-to-end
+// test asks for 0.5 % of either.  This order is the one furthest inside that bar
+// (+0.29 % and -0.19 %); another may fail the test without being wrong.
 __device__ __forceinline__ float2 inv_pair(float2 xu, float2 xn, float2 e) {
     const float P = __fadd_rn(xu.x, xn.y), Q = __fsub_rn(xu.y, xn.x);
     return make_float2(__fmaf_rn(e.y, Q, __fmul_rn(e.x, P)), __fmaf_rn(-e.y, P, __fmul_rn(e.x, Q)));
@@ -850,13 +856,18 @@ template <int N, int P>
 static size_t rows_inv_smem() { return 8 * (size_t)N * P; }
 
 // Pairs per block.  A block is at least one warp, where a barrier costs least.
-// Measured on square grids (us per pass, L2-warm; rows forward from the map):
-//   rows forward   P = 1 / 2 / 4   64: - / 6.1 / 5.3   256: 7.6 / 6.7 / 7.3   512: 7.9 / 7.1 / 8.2   1024: 11.4 / 10.1 / 10.7
-//                                  2048: 22.9 / 23.9 / 28.4   4096: 84 / 102
-//   columns        P = 1 / 2 / 4   256: 5.2 / 5.3 / 5.2   512: 6.6 / 5.5 / 6.5   1024: 15.7 / 13.1 / 11.9
-//                                  2048: 54 / 43 / 34   4096: 208 / 153
-//   rows inverse   P = 1 / 2 / 4   256: 2.3 / 2.7 / 3.4   512: 3.5 / 3.2 / 3.9   1024: 5.4 / 6.4 / 7.3
-//                                  2048: 14.7 / 18.6 / 26.5   4096: 69 / 103
+// Measured on square grids (us per pass, L2-warm; rows forward from the map; below 256
+// one pair is less than a warp):
+//   rows forward   P = 1 / 2 / 4   64: - / 6.0 / 6.4   128: - / 6.5 / 6.9   256: 7.7 / 6.8 / 7.4   512: 7.9 / 7.1 / 8.2
+//                                  1024: 11.4 / 10.1 / 10.7   2048: 22.9 / 23.9 / 28.4   4096: 84 / 102
+//   columns        P = 1 / 2 / 4   64: - / 3.5 / 3.2   128: - / 5.1 / 4.8   256: 5.2 / 5.3 / 5.2   512: 6.6 / 5.5 / 6.5
+//                                  1024: 15.7 / 13.1 / 11.9   2048: 54 / 43 / 34   4096: 208 / 153
+//   rows inverse   P = 1 / 2 / 4   64: - / 1.8 / 2.5   128: - / 2.1 / 3.1   256: 2.2 / 2.7 / 3.3   512: 3.5 / 3.2 / 3.9
+//                                  1024: 5.4 / 6.4 / 7.3   2048: 14.7 / 18.6 / 26.5   4096: 69 / 103
+// (P = 8: rows forward 7.4 and 8.3, columns 3.3 and 4.9, rows inverse 2.4 and 3.2 at 64
+// and 128.)  Side 64 keeps four pairs in the rows forward, 0.4 us a pass more than two:
+// eight steps at 2,003 cells take 309 us, 307 with two, and the overflow's block sums
+// would be grouped otherwise.
 // The column pass reads and writes runs of 16 P bytes; large grids, where L2 traffic
 // counts, want long ones, small grids a block for every SM.  Side 4096 has room for
 // P = 2 (two arrays of 8 N P bytes).
