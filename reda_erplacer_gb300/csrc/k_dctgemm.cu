@@ -26,8 +26,9 @@
 // thread) and store it meanwhile.  Every mbarrier wait is bounded (status bit
 // kStatusWaitTimeout).
 //
-// What bounds it: up to 1024^2 the operands' way from L2 (0.3 us per 32 columns of K
-// with 24 KB per CTA and step, 10 TB/s over 128 CTAs); at 2048^2 the tensor cores with
+// What bounds it: up to 1024^2 the latency of the operands' way from L2 through the ring
+// (0.3 us per 32 columns of K with 24 KB per CTA and step; at 1024^2 the L2 is at 14 to
+// 19 % of its rate and the tensor pipe active for 12 to 56 % of the cycles); at 2048^2 the tensor cores with
 // their last wave (2.5 waves of 128 x 256 tiles for three maps).  Measured against one
 // CTA of 128 threads per tile with a shared-memory transpose in its epilogue, us per
 // solve on the device: 2048^2 BF16x3 with the potential 476 -> 317, TF32 290 -> 229;
